@@ -283,10 +283,9 @@ int rnj_distance_matrix_host_ex(rnj_ctx *ctx, const char *chars, int n, int L, s
 /* Many alignments computed together.  The triangle tiles of every alignment
  * added form one device work list, ordered by decreasing cost, that one
  * persistent launch per kernel family consumes (the tensor-core kernel for DNA,
- * the bit-plane kernel for protein and -f alignments), followed by the
- * saturation fix-up; the launch sequence is captured once, at creation, in a
- * CUDA graph, and a run only uploads the descriptors and work lists the graph
- * reads.  For a stream of alignments this replaces one driver call per
+ * the bit-plane kernel for -f alignments and large alphabets), followed by the
+ * saturation fix-up; a run uploads the descriptors and work lists that these
+ * read.  For a stream of alignments this replaces one driver call per
  * alignment (JCdistance / KimuraDistance per input, or per bootstrap replicate
  * of main.cpp:519-532).  Capacities bound the alignments and the total tiles
  * (128 x 128 pairs each, (ceil(n/128)+1)*ceil(n/128)/2 per alignment).  The
@@ -324,7 +323,7 @@ int rnj_batch_size(rnj_batch *batch, int *alignments, long long *tiles);
  * alignments had a tuned entry (each one's tile-order band comes from it).
  * Either pointer may be NULL. */
 int rnj_batch_tuning(rnj_batch *batch, int *ring_depth, int *tuned_alignments);
-/* Forgets the alignments (frees outputs still owned by the batch); the graph stays. */
+/* Forgets the alignments (frees outputs still owned by the batch). */
 int rnj_batch_clear(rnj_batch *batch);
 int rnj_batch_destroy(rnj_batch *batch);
 

@@ -396,7 +396,7 @@ class Context:
 
 class Batch:
     """Many alignments in one persistent pass (rnj_batch): a device work list of
-    all their tiles, consumed by graph-captured persistent kernels."""
+    all their tiles, consumed by persistent kernels."""
 
     def __init__(self, ctx: Context, max_alignments: int = 1024, max_tiles: int = 1 << 16):
         h = ctypes.c_void_p()

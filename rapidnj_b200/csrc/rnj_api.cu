@@ -73,17 +73,46 @@ int encode_planes_map(Packed &p) {
   return RNJ_OK;
 }
 
-// 3-D map over the K-blocked FP4 features: (128 bytes, Np rows, 4 * Lk / 256
-// blocks), box 128 x 128 x 1 = one contiguous 16 KB run, 128-byte swizzle (the
-// layout the tcgen05 shared-memory descriptors expect).
+namespace {
+
+// A map over the K-blocked FP4 features: (128 bytes, Np rows, Lk / 256 K blocks,
+// feature blocks); a box is `blocks` K blocks of `rows` rows, each one contiguous
+// run, 128-byte swizzled (the layout the tcgen05 shared-memory descriptors
+// expect).
+int encode_feature_box(const Packed &p, int rows, int blocks, CUtensorMap *map) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return set_error(RNJ_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  const cuuint64_t seg = (cuuint64_t)p.Lk / 256, slab = (cuuint64_t)p.Np * 128;
+  cuuint64_t dims[4] = {128, (cuuint64_t)p.Np, seg, (cuuint64_t)p.nfb};
+  cuuint64_t strides[3] = {128, slab, slab * seg};
+  cuuint32_t box[4] = {128, (cuuint32_t)rows, (cuuint32_t)blocks, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, p.feat, dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return set_error(RNJ_ERR_CUDA, "cuTensorMapEncodeTiled (features) failed (" +
+                                       std::to_string((int)r) + ")");
+  return RNJ_OK;
+}
+
+}  // namespace
+
 int encode_features_map(Packed &p) {
+  const int rc = encode_feature_box(p, kTile, 2, &p.fmap_a);
+  return rc != RNJ_OK ? rc : encode_feature_box(p, kTile / 2, 2, &p.fmap_b);
+}
+
+// (128 bytes, Np rows, nfb * Lk / 256 blocks), box 128 x 128 x 1 = one contiguous
+// 16 KB run.
+int encode_block_map(const Packed &p, CUtensorMap *map) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return set_error(RNJ_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
   cuuint64_t dims[3] = {128, (cuuint64_t)p.Np, (cuuint64_t)p.nfb * (p.Lk / 256)};
   cuuint64_t strides[2] = {128, (cuuint64_t)p.Np * 128};
   cuuint32_t box[3] = {128, (cuuint32_t)kTile, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(&p.fmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, p.feat, dims, strides, box, estr,
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, p.feat, dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
@@ -153,7 +182,12 @@ EpiParams epi_params_for(const Packed &p, int model) {
 AlnDesc desc_for(const Packed &p, const EpiParams &ep) {
   AlnDesc d;
   memset(&d, 0, sizeof(d));
-  d.map = is_tc_kind(p.kind) ? p.fmap : p.tmap;
+  if (is_tc_kind(p.kind)) {
+    d.map_a = p.fmap_a;
+    d.map_b = p.fmap_b;
+  } else {
+    d.map = p.tmap;
+  }
   d.out = ep.out;
   d.counts = ep.counts;
   d.ld = ep.ld;
@@ -433,6 +467,10 @@ int run_tc_single(rnj_ctx *ctx, const Packed &p, const EpiParams &ep, int epi_mo
   const TuneParams tp = tune_lookup(p.n, p.L, p.type, p.flags);
   AlnDesc d = desc_for(p, ep);
   d.band = tp.tile_band;
+  if (epi_mode == EPI_COUNTS || !tc_fused_form(p, tp)) {
+    const int rc = encode_block_map(p, &d.map);
+    if (rc != RNJ_OK) return rc;
+  }
   // Pageable source: the copy is taken before the call returns, so the stack
   // descriptor may go out of scope.
   RNJ_CUDA(cudaMemcpyAsync(ctx->d_desc, &d, sizeof(d), cudaMemcpyHostToDevice, ctx->stream),
@@ -444,7 +482,7 @@ int run_tc_single(rnj_ctx *ctx, const Packed &p, const EpiParams &ep, int epi_mo
              "tensor-core kernel");
     return RNJ_OK;
   }
-  return run_tc_distances(ctx, p, ep, ctx->d_desc, nullptr, ntiles, ctx->stream, tp);
+  return run_tc_distances(ctx, p, ep, ctx->d_desc, ctx->stream, tp);
 }
 
 // Waits for the context's stream and reports (and clears) the sticky device
@@ -560,13 +598,12 @@ int ensure_packed(rnj_ctx *ctx, long long tiles) {
 }
 
 int run_tc_distances(rnj_ctx *ctx, const Packed &p, const EpiParams &ep, const AlnDesc *d_desc,
-                     const WorkItem *d_items, long long nitems, cudaStream_t s,
-                     const TuneParams &tp) {
-  if (tp.tc_epilogue == 0 && p.L <= kMaxFusedColumns) {
+                     cudaStream_t s, const TuneParams &tp) {
+  if (tc_fused_form(p, tp)) {
     // Counts and transform in one launch (rnj_tcf.cu).
     mark(ctx, 1, 0);
-    RNJ_CUDA(launch_tc_fused(d_desc, d_items, nullptr, (int)nitems, 0, (int)nitems,
-                             (int)std::min<long long>(nitems, ctx->num_sms),
+    const int count = (int)pair_items(tiles_of(p.n));
+    RNJ_CUDA(launch_tc_fused(d_desc, nullptr, 0, count,
                              fused_variant_for(ep.model, ep.type, ep.compat_wrap, 0), s,
                              tp.tc_stages),
              "fused tensor-core kernel");
@@ -574,9 +611,10 @@ int run_tc_distances(rnj_ctx *ctx, const Packed &p, const EpiParams &ep, const A
     mark(ctx, 2, 0);
     return RNJ_OK;
   }
-  int rc = ensure_packed(ctx, std::min<long long>(nitems, kTcChunkTiles));
+  const long long ntiles = tri_tiles(tiles_of(p.n));
+  int rc = ensure_packed(ctx, std::min<long long>(ntiles, kTcChunkTiles));
   if (rc != RNJ_OK) return rc;
-  return run_tc_chunks(ctx, d_desc, d_items, nitems, ctx->d_packed, s, tp.transform_ctas,
+  return run_tc_chunks(ctx, d_desc, nullptr, ntiles, ctx->d_packed, s, tp.transform_ctas,
                        tp.tc_stages);
 }
 

@@ -2,8 +2,8 @@
 // triangle tiles of every alignment in the batch, ordered by decreasing cost,
 // consumed by one persistent launch per kernel family (the tcgen05 kernel for
 // DNA, the bit-plane kernel for protein and -f alignments) and a fix-up over the
-// flagged tiles.  The launch sequence is captured once in a CUDA graph; a run
-// only uploads the descriptors and work lists the graph's kernels read.
+// flagged tiles.  A run uploads the descriptors and work lists and launches the
+// kernels that have items.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
@@ -43,7 +43,7 @@ struct rnj_batch {
   rnj_ctx *ctx = nullptr;
   int cap_aln = 0;
   long long cap_tiles = 0;
-  cudaStream_t stream = nullptr;  // capture / launch stream (non-blocking)
+  cudaStream_t stream = nullptr;  // launch stream (non-blocking)
   cudaEvent_t ev_ready = nullptr, ev_uploaded = nullptr, ev_done = nullptr;
   bool uploaded_pending = false;
   // device
@@ -56,9 +56,6 @@ struct rnj_batch {
   AlnDesc *h_descs = nullptr;
   WorkItem *h_items_tc = nullptr, *h_items_pc = nullptr;
   int *h_ints = nullptr;
-  // graph
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
   std::vector<Entry> entries;
   long long tiles_used = 0;
   bool join = true;  // make the context stream wait for each run's completion
@@ -86,8 +83,6 @@ void free_batch(rnj_batch *b) {
     if (e.owns_aln) rnj_aln_destroy(e.aln);
   }
   for (void *a : b->arenas) cudaFreeAsync(a, b->ctx->stream);
-  if (b->exec) cudaGraphExecDestroy(b->exec);
-  if (b->graph) cudaGraphDestroy(b->graph);
   cudaFree(b->d_descs);
   cudaFree(b->d_items_tc);
   cudaFree(b->d_items_pc);
@@ -103,36 +98,6 @@ void free_batch(rnj_batch *b) {
   if (b->ev_done) cudaEventDestroy(b->ev_done);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
-}
-
-// Captures: clear scratch -> the fused tensor-core kernel over every
-// tensor-core item (counts and transform, per-item model) -> popcount kernel ->
-// fix-up.
-int capture_graph(rnj_batch *b) {
-  const int sms = b->ctx->num_sms;
-  RNJ_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-  cudaError_t e = cudaMemsetAsync(b->d_max, 0, sizeof(int) * b->cap_aln, b->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b->d_flags, 0, sizeof(int) * b->cap_tiles, b->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(b->d_ints + 2, 0, 2 * sizeof(int), b->stream);
-  if (e == cudaSuccess)
-    e = launch_tc_fused(b->d_descs, b->d_items_tc, b->d_ints + 0, 0, 0, (int)b->cap_tiles, sms,
-                        FUSED_ANY, b->stream);
-  if (e == cudaSuccess)
-    e = launch_count_batch(b->d_descs, b->d_items_pc, b->d_ints + 1, b->d_ints + 2, sms, EPI_DIST,
-                           b->stream);
-  if (e == cudaSuccess)
-    e = launch_fixup_batch(b->d_descs, b->d_items_tc, b->d_ints + 0, b->d_items_pc, b->d_ints + 1,
-                           sms * 4, b->stream);
-  cudaGraph_t g = nullptr;
-  cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
-  if (e != cudaSuccess) {
-    if (g) cudaGraphDestroy(g);
-    return cuda_error(e, "batch graph capture");
-  }
-  if (e2 != cudaSuccess) return cuda_error(e2, "end capture");
-  b->graph = g;
-  RNJ_CUDA(cudaGraphInstantiate(&b->exec, g, 0), "graph instantiate");
-  return RNJ_OK;
 }
 
 }  // namespace
@@ -165,11 +130,6 @@ int rnj_batch_create(rnj_ctx *ctx, int max_alignments, long long max_tiles, rnj_
   if (e != cudaSuccess) {
     free_batch(b);
     return cuda_error(e, "batch allocation");
-  }
-  int rc = capture_graph(b);
-  if (rc != RNJ_OK) {
-    free_batch(b);
-    return rc;
   }
   *out = b;
   return RNJ_OK;
@@ -427,27 +387,28 @@ int rnj_batch_run(rnj_batch *b) {
       }
     }
     b->tuned_alns = tuned;
-    // The graph's launch holds the deepest ring; the run's depth travels in
-    // the first descriptor (no re-capture).
     b->tc_stages = depth;
-    if (na > 0) b->h_descs[0].stages = depth;
   }
+  // Bit-plane items as row-major tiles, tensor-core ones as row pairs in the banded
+  // order of their bucket's band height (PairWalk's; consecutive items go to
+  // consecutive CTA pairs, which then share row tiles in L2; never more items
+  // than tiles).
+  int variant = -1;  // the transform of every tensor-core item, FUSED_ANY if they differ
   for (int oi = 0; oi < na; ++oi) {
     const int a = order[oi];
     const Entry &en = b->entries[a];
-    const bool tc = is_tc_kind(en.aln->p.kind);
-    // tensor-core triangles in the banded order of their bucket's band
-    // height (consecutive items go to consecutive CTAs, which then share row
-    // tiles in L2); full-square and bit-plane items in row-major order
-    const bool banded = tc && !b->h_descs[a].full;
-    const int nt = b->h_descs[a].nt;
-    for (long long t = 0; t < en.ntiles; ++t) {
-      WorkItem w;
-      w.aln = a;
-      w.tile = banded ? banded_tile((int)t, nt, bands[a]) : (int)t;
-      if (tc) b->h_items_tc[ntc++] = w;
-      else b->h_items_pc[npc++] = w;
+    const AlnDesc &da = b->h_descs[a];
+    if (!is_tc_kind(en.aln->p.kind)) {
+      for (long long t = 0; t < en.ntiles; ++t) b->h_items_pc[npc++] = WorkItem{a, (int)t};
+      continue;
     }
+    const int v = fused_variant_for(da.model, da.type, da.compat, 0);
+    variant = variant < 0 || variant == v ? v : (int)FUSED_ANY;
+    const int nt = da.nt, band = 2 * pair_band(bands[a]);
+    for (int r0 = 0; r0 < nt; r0 += band)
+      for (int tj = r0; tj < nt; ++tj)
+        for (int ti = r0; ti <= tj && ti < r0 + band; ti += 2)
+          b->h_items_tc[ntc++] = WorkItem{a, tri_index(ti, tj, nt)};
   }
   b->h_ints[0] = (int)ntc;
   b->h_ints[1] = (int)npc;
@@ -466,13 +427,32 @@ int rnj_batch_run(rnj_batch *b) {
     RNJ_CUDA(cudaMemcpyAsync(b->d_items_pc, b->h_items_pc, sizeof(WorkItem) * npc,
                              cudaMemcpyHostToDevice, b->stream),
              "work list upload");
-  RNJ_CUDA(cudaMemcpyAsync(b->d_ints, b->h_ints, 2 * sizeof(int), cudaMemcpyHostToDevice, b->stream),
+  b->h_ints[2] = b->h_ints[3] = 0;  // the item counter and the error word
+  RNJ_CUDA(cudaMemcpyAsync(b->d_ints, b->h_ints, 4 * sizeof(int), cudaMemcpyHostToDevice, b->stream),
            "count upload");
-  RNJ_CUDA(cudaMemsetAsync(b->d_ints + 3, 0, sizeof(int), b->stream), "error clear");
   RNJ_CUDA(cudaEventRecord(b->ev_uploaded, b->stream), "upload event");
   b->uploaded_pending = true;
   b->host_max_valid = false;
-  RNJ_CUDA(cudaGraphLaunch(b->exec, b->stream), "graph launch");
+  if (na > 0) {
+    // Maxima and flags cleared, the fused kernel over the tensor-core items (a
+    // mixed list by each item's descriptor, any other by its own variant, whose
+    // epilogue is leaner: 18k against 26k cycles a K2P tile), the bit-plane
+    // kernel, the fix-up.
+    const int sms = ctx->num_sms;
+    RNJ_CUDA(cudaMemsetAsync(b->d_max, 0, sizeof(int) * na, b->stream), "max clear");
+    RNJ_CUDA(cudaMemsetAsync(b->d_flags, 0, sizeof(int) * b->tiles_used, b->stream), "flag clear");
+    if (ntc > 0)
+      RNJ_CUDA(launch_tc_fused(b->d_descs, b->d_items_tc, 0, (int)ntc, variant, b->stream,
+                               b->tc_stages),
+               "fused tensor-core kernel");
+    if (npc > 0)
+      RNJ_CUDA(launch_count_batch(b->d_descs, b->d_items_pc, b->d_ints + 1, b->d_ints + 2, sms,
+                                  EPI_DIST, b->stream),
+               "count kernel");
+    RNJ_CUDA(launch_fixup_batch(b->d_descs, b->d_items_tc, b->d_ints + 0, b->d_items_pc,
+                                b->d_ints + 1, sms * 4, b->stream),
+             "fix-up kernel");
+  }
   RNJ_CUDA(cudaEventRecord(b->ev_done, b->stream), "done event");
   // Later work on the context stream (copies, new packs) sees the results.
   if (b->join) RNJ_CUDA(cudaStreamWaitEvent(ctx->stream, b->ev_done, 0), "join");

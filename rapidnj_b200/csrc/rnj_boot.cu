@@ -80,7 +80,7 @@ extern "C" int rnj_bootstrap(rnj_ctx *ctx, const void *d_chars, int n, int L, si
   const long long rep_tiles = tri_tiles(tiles_of(n));
   int chunk = (int)std::max<long long>(1, std::min<long long>(R, (1LL << 30) / rep_bytes));
   chunk = (int)std::min<long long>(chunk, std::max<long long>(1, (8LL * kTcChunkTiles) / rep_tiles));
-  // The context keeps the batch (its graph and buffers) for later calls of the
+  // The context keeps the batch (its buffers) for later calls of the
   // same or a smaller size.
   int rc = RNJ_OK;
   if (!ctx->boot || ctx->boot_aln < chunk || ctx->boot_tiles < (long long)chunk * rep_tiles) {

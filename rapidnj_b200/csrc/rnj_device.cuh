@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "rnj_logtab.h"
+#include "rnj_logtab_q.h"
 
 namespace rnj {
 
@@ -146,54 +147,59 @@ __device__ __forceinline__ double ln_table(double x) {
   return __fma_rn(dk, kLn2Hi, __dadd_rn(__fma_rn(dk, kLn2Lo, lnF), p));
 }
 
-// -ln(x) / 4, the K2P fast path's logarithm, with the table read from `tab`
-// (a copy of c_log_tab in shared memory, each entry scaled by -1/4: a warp's
-// 32 random entries are one shared-memory request instead of up to 16 L1
-// lines) and k turned into a double by the 2^52 bias (an integer add and a
-// double subtraction, both exact, instead of a conversion).  The arithmetic
-// is ln_table's with every operand scaled by a power of two: r' = -r / 4 (the
-// table's -1/(4F)), Horner coefficients c_k (-4)^k, so the k-th Horner value
-// is (-4)^k times ln_table's and the product with r' is -1/4 of its; ln F and
-// ln 2 scaled by -1/4.  Rounding to nearest commutes with a power-of-two
-// scale (no operand comes near overflow or underflow), so the result is
-// exactly -ln_table(x) / 4, with ln_table's error bound divided by 4.
-constexpr double kNegQuarterLn2Hi = -0.25 * kLn2Hi, kNegQuarterLn2Lo = -0.25 * kLn2Lo;
-__device__ __forceinline__ double neg_quarter_ln_table_k(double x, const double2 *tabq) {
-  const long long bits = __double_as_longlong(x);
-  const int ebits = (int)((bits >> 52) & 0x7FF);  // k + 1023
-  const int j = (int)((bits >> 45) & 127);
-  const double m = __longlong_as_double((bits & 0x000FFFFFFFFFFFFFLL) | 0x3FF0000000000000LL);
-  const double F = __longlong_as_double(0x3FF0000000000000LL | ((long long)j << 45));
-  const double2 e = tabq[j];  // {-ln F / 4, -1 / (4 F)}
-  const double r = __dmul_rn(__dsub_rn(m, F), e.y);
-  double p = (-1.0 / 6.0) * -1024.0;
-  p = __fma_rn(p, r, 0.2 * 256.0);
-  p = __fma_rn(p, r, -0.25 * -64.0);
-  p = __fma_rn(p, r, (1.0 / 3.0) * 16.0);
-  p = __fma_rn(p, r, -0.5 * -4.0);
-  p = __fma_rn(p, r, 1.0);
-  p = __dmul_rn(p, r);
-  // 2^52 + ebits, exactly, minus 2^52 + 1023: the double k (|k| < 2^11).
+// -ln(x) / 4 for the fused epilogue, x in [2^-126, 1]: table-driven reduction
+// (Tang, as above) over 128 intervals of [kLnLow, 2 kLnLow), kLnLow = 0.70703125.
+// x = 2^k z with z in that range, j = z's interval, inv = the table's double near
+// 1 / midpoint, r = z inv - 1 in one fused multiply-add (|r| <= 2^-8, below 2^-7
+// in the interval above 1), ln x = k ln 2 - ln inv + ln(1 + r) with the series to
+// r^5, every constant scaled by -1/4.  t2: the high word less that of kLnLow, plus
+// 2^29, whose fields are the biased k (bits 20 ..) and j; for x = 0 and negative x
+// bit 31 is set, for a NaN bit 30 (callers test both).  8 double operations,
+// against 12 of ln_table.
+//
+// tab: this lane's copy of c_log_tab_q in shared memory.  There are eight, 16
+// bytes apart in every 128-byte entry, one for each lane of a quarter warp, so
+// that the 16-byte reads of random entries never meet on a bank: with one copy
+// the conflicts were a third of what the load/store pipe did in the kernel.
+//
+// The two intervals that meet at 1 have inv = 1, so r = z - 1 is exact there
+// and the error below is relative: of -ln(x) / 4,
+//   series remainder   r^5 / 6 < 2^-42.5 next to 1; elsewhere r^6 / 6 < 2^-50.5
+//                      against |ln x| >= 2^-8 (2^-44.5 against ln 2 / 2 above 1)
+//   ln inv             2^-55 against |ln x| >= 2^-8
+//   everything else    a few 2^-53
+// together below 2^-42.  x = 1 gives exactly -0.0 (0 * (-1/4) and -0.0 added to
+// -0.0), the reference's value for identical pairs.
+constexpr int kLnCopies = 8;
+__device__ __forceinline__ double neg_quarter_ln(double x, const double2 *tab, uint32_t &t2) {
+  t2 = (uint32_t)__double2hiint(x) - (kLnOff - 0x20000000u);
+  const double2 e = *reinterpret_cast<const double2 *>(reinterpret_cast<const char *>(tab) +
+                                                       ((t2 >> 6) & 0x3F80u));
+  const double z = __hiloint2double((int)((t2 & 0xFFFFFu) + kLnOff), __double2loint(x));
+  const double r = __fma_rn(z, e.y, -1.0);
+  // 2^52 + biased k, exactly, less 2^52 + 512: the double k
   const double dk =
-      __dsub_rn(__hiloint2double(0x43300000, ebits), 4503599627370496.0 + 1023.0);
-  return __fma_rn(dk, kNegQuarterLn2Hi, __dadd_rn(__fma_rn(dk, kNegQuarterLn2Lo, e.x), p));
+      __dsub_rn(__hiloint2double(0x43300000, (int)(t2 >> 20)), 4503599627370496.0 + 512.0);
+  const double s = __fma_rn(dk, kNegQuarterLn2, e.x);
+  double q = -1.0 / 20.0;
+  q = __fma_rn(q, r, 1.0 / 16.0);
+  q = __fma_rn(q, r, -1.0 / 12.0);
+  q = __fma_rn(q, r, 0.125);
+  q = __fma_rn(q, r, -0.25);
+  return __fma_rn(q, r, s);
 }
 
-// The double of an integer 0 <= v < 2^32: 2^52 + v has v in its low mantissa
-// bits, so the subtraction of 2^52 is exact.
-__device__ __forceinline__ double u32_to_double(uint32_t v) {
-  return __dsub_rn(__hiloint2double(0x43300000, (int)v), 4503599627370496.0);
-}
-
-// y rounded to 24 significant bits, to nearest, in double arithmetic: Veltkamp
-// splitting with C = 2^29 + 1 (Dekker 1971): g = fl(C y), h = fl(g - fl(g - y))
-// keeps the 53 - 29 = 24 leading bits of y rounded to nearest (Boldo 2006; a
-// tie may round either way).  For 2^-126 <= |y| < 2^127 that is (double)(float)y
-// unless y lies exactly halfway between two floats.
-__device__ __forceinline__ double round_to_float_bits(double y) {
-  const double g = __dmul_rn(y, 536870913.0);
-  return __dsub_rn(g, __dsub_rn(g, y));
-}
+// Whether a double within m * 2^-53 (relative) of dd >= 0 could round to another
+// float than dd: the 29 bits of dd's significand below the float's lie within m
+// of the midpoint 2^28 (m < 2^28).  The top three bits of the low word drop out
+// of the product by 8.
+struct RoundCheck {
+  uint32_t k1, k2;
+  __device__ __forceinline__ explicit RoundCheck(uint32_t m) : k1(8u * m - 0x80000000u), k2(16u * m) {}
+  __device__ __forceinline__ bool undecided(double dd) const {
+    return (uint32_t)__double2loint(dd) * 8u + k1 < k2;
+  }
+};
 
 // Valid-site count as the fast protein estimator reports it for L % 128 == 0
 // (bitDistanceProtein.cpp:15-16,59): padded length minus the gaps counted over
@@ -214,18 +220,6 @@ __device__ __forceinline__ unsigned long long protein_fast_valid(unsigned long l
 // dd - eps and dd + eps round to the same float so does d_ref.
 __device__ __forceinline__ float neg_log_checked(double c, double arg) {
   const double dd = __dmul_rn(-c, ln_table(arg));
-  const double eps = __dmul_rn(0x1p-49, __dadd_rn(1.0, __dmul_rn(4.0, dd)));
-  const float lo = __double2float_rn(__dsub_rn(dd, eps));
-  const float hi = __double2float_rn(__dadd_rn(dd, eps));
-  return __float_as_int(lo) == __float_as_int(hi) ? lo : __int_as_float(0x7fc00000);
-}
-
-// neg_log_checked with the table read from `tabq`, the shared-memory copy scaled
-// by -1/4 (neg_quarter_ln_table_k): ln_table(arg) is exactly -4 times that value
-// (a power-of-two scale), so dd, the check and the result are neg_log_checked's
-// bit for bit.
-__device__ __forceinline__ float neg_log_checked_tab(double c, double arg, const double2 *tabq) {
-  const double dd = __dmul_rn(c, __dmul_rn(4.0, neg_quarter_ln_table_k(arg, tabq)));
   const double eps = __dmul_rn(0x1p-49, __dadd_rn(1.0, __dmul_rn(4.0, dd)));
   const float lo = __double2float_rn(__dsub_rn(dd, eps));
   const float hi = __double2float_rn(__dadd_rn(dd, eps));
@@ -299,7 +293,7 @@ __device__ __forceinline__ float jc_distance(unsigned long long total,
 }
 
 // JCdistance.cpp:177-183 from the float p (0 when valid is 0).
-__device__ __forceinline__ float jc_of_q(double q, double b, const double2 *tabq = nullptr);
+__device__ __forceinline__ float jc_of_q(double q, double b);
 
 __device__ __forceinline__ float jc_of_p(float distance, double b) {
   return jc_of_q(__ddiv_rn((double)distance, b), b);
@@ -316,13 +310,12 @@ __device__ __forceinline__ double div_by_b(double p, double b, double inv_b) {
   return __fma_rn(__fma_rn(-q0, b, p), inv_b, q0);
 }
 
-// JCdistance.cpp:177-183 from q = (double)p / b.  tabq: the logarithm table in
-// shared memory (neg_log_checked_tab), or null for the global one.
-__device__ __forceinline__ float jc_of_q(double q, double b, const double2 *tabq) {
+// JCdistance.cpp:177-183 from q = (double)p / b.
+__device__ __forceinline__ float jc_of_q(double q, double b) {
   if (q >= 1.0) return -1.0f;
   const double arg = __dsub_rn(1.0, q);
   if (arg == 1.0) return __double2float_rn(__dmul_rn(-b, 0.0));  // -0.0, as the reference
-  const float fast = tabq ? neg_log_checked_tab(b, arg, tabq) : neg_log_checked(b, arg);
+  const float fast = neg_log_checked(b, arg);
   if (fast == fast) return fast;
   return neg_log_slow(b, arg);
 }
@@ -382,30 +375,6 @@ __device__ __forceinline__ float k2p_distance(unsigned long long ts_count,
   return k2p_two_logs(a, b);
 }
 
-// The K2P distance of k2p_distance for 1 <= n < 2^24 (the fused kernel's
-// counts), without branches, so that the pairs of a group interleave: the
-// saturated (-1) and identical (-0.0) cases and the one-logarithm value are
-// computed for every pair and selected.  *slow is set when the rounding check
-// cannot decide (about one pair in 10^6-10^7); the caller then evaluates
-// k2p_distance for that pair.  n == 0 gives -1 like k2p_distance.
-__device__ __forceinline__ float k2p_decide(uint32_t P, uint32_t Q, uint32_t n, bool &slow) {
-  const double rn = recip_nr(n == 0 ? 1u : n);
-  const float ts = __double2float_rn(__dmul_rn((double)P, rn));
-  const float tv = __double2float_rn(__dmul_rn((double)Q, rn));
-  const double a = __dsub_rn(__dsub_rn(1.0, __dmul_rn(2.0, (double)ts)), (double)tv);
-  const double b = __dsub_rn(1.0, __dmul_rn(2.0, (double)tv));
-  const bool sat = (n == 0) | (__double2float_rn(a) <= 0.0f) | (__double2float_rn(b) <= 0.0f);
-  const bool same = (P | Q) == 0;
-  // a, b in (0, 1] unless saturated: ln_table's argument stays positive.
-  const double x = sat ? 1.0 : __dmul_rn(__dmul_rn(a, a), b);
-  const double dd = __dmul_rn(-0.25, ln_table(x));
-  const double eps = __dmul_rn(0x1p-49, __dadd_rn(1.0, __dmul_rn(4.0, dd)));
-  const float lo = __double2float_rn(__dsub_rn(dd, eps));
-  const float hi = __double2float_rn(__dadd_rn(dd, eps));
-  slow = !sat && !same && (__float_as_int(lo) != __float_as_int(hi));
-  return sat ? -1.0f : (same ? -0.0f : lo);
-}
-
 // 1 / d for an integer 1 <= d < 2^16 given as a float: one Newton-Raphson step
 // r0 + r0 (1 - d r0) from the fast reciprocal (|d r0 - 1| <= 2^-21).  1 - d r0
 // is exact as a fused multiply-add (d r0 has at most 40 significant bits and
@@ -426,50 +395,58 @@ __device__ __forceinline__ float recip16(float d) {
 // would need M | num < 2^16), so q is the correctly rounded quotient: the
 // reference's (float)((double)num / (double)d) and (float)num / (float)d (the
 // double quotient is no midpoint either, so its float rounding agrees).
-__device__ __forceinline__ float quotient16(uint32_t num, float d, float y) {
-  const float fnum = __fsub_rn(__uint_as_float(0x4B000000u | num), 8388608.0f);
+// A numerator scaled by a power of two gives the quotient scaled by it (every
+// step commutes with the scale), which the fused epilogue uses for 4 P and 2 Q.
+__device__ __forceinline__ float quotient_of(float fnum, float d, float y) {
   const float q0 = __fmul_rn(fnum, y);
   return __fmaf_rn(__fmaf_rn(-q0, d, fnum), y, q0);
 }
+__device__ __forceinline__ float quotient16(uint32_t num, float d, float y) {
+  return quotient_of(__fsub_rn(__uint_as_float(0x4B000000u | num), 8388608.0f), d, y);
+}
 
-// k2p_decide for 16-bit counts (the fused kernel): P, Q, n < 2^16 given as
-// integers packed by the epilogue.  The same decision and result, computed
-// with fewer conversions:
-//   * the floats of P, Q and n by the 2^23 bias; ts, tv = quotient16, the
-//     reference's float quotients, converted to double exactly;
-//   * temp1 = (float)a <= 0 exactly when a <= 0: a and b are sums of doubles
-//     of floats in [0, 1] with at most 24 significant bits and exponents above
-//     -17, so a nonzero a or b exceeds 2^-70 in magnitude and its float is not 0;
-//   * neg_quarter_ln_table_k for -ln(x) / 4 (tab: the table in shared memory,
-//     scaled by -1/4).
-__device__ __forceinline__ float k2p_decide16(uint32_t P, uint32_t Q, uint32_t n, bool &slow,
-                                              const double2 *tab) {
-  const uint32_t nn = n == 0 ? 1u : n;
-  const float fn = __fsub_rn(__uint_as_float(0x4B000000u | nn), 8388608.0f);
-  const float y = recip16(fn);
-  const double ts = (double)quotient16(P, fn, y);
-  const double tv = (double)quotient16(Q, fn, y);
-  // fl(1 - 2 ts) as one fused multiply-add: 2 ts is exact, so both forms are
-  // the exact 1 - 2 ts rounded once (the reference's double arithmetic).
-  const double a = __dsub_rn(__fma_rn(-2.0, ts, 1.0), tv);
-  const double b = __fma_rn(-2.0, tv, 1.0);
-  const bool sat = (n == 0) | (a <= 0.0) | (b <= 0.0);
-  const bool same = (P | Q) == 0;
-  const double x = sat ? 1.0 : __dmul_rn(__dmul_rn(a, a), b);
-  const double dd = neg_quarter_ln_table_k(x, tab);  // -ln(x) / 4, exactly as scaled
-  // eps = 2^-49 (1 + 4 dd), one fused multiply-add (rounded once, as close to
-  // the bound as the three-operation form)
-  const double eps = __fma_rn(0x1p-47, dd, 0x1p-49);
-  const float lo = __double2float_rn(__dsub_rn(dd, eps));
-  const float hi = __double2float_rn(__dadd_rn(dd, eps));
-  slow = !sat && !same && (__float_as_int(lo) != __float_as_int(hi));
-  return sat ? -1.0f : (same ? -0.0f : lo);
+// Two floats in one 64-bit register, and the packed operations on them (each
+// half rounded like the scalar operation): the float part of the fused epilogue
+// takes two pairs at a time.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 x, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// recip16 and quotient_of for two pairs; nd = -d.
+__device__ __forceinline__ f32x2 recip16_2(f32x2 d, f32x2 nd) {
+  float a, b;
+  unpack2(d, a, b);
+  const f32x2 r0 = pack2(rcp_approx(a), rcp_approx(b));
+  return fma2(r0, fma2(nd, r0, pack2(1.0f, 1.0f)), r0);
+}
+__device__ __forceinline__ f32x2 quotient_of_2(f32x2 num, f32x2 nd, f32x2 y) {
+  const f32x2 q0 = mul2(num, y);
+  return fma2(fma2(q0, nd, num), y, q0);
 }
 
 // KimuraDistance.cpp:322-338 with the Dayhoff table of KimuraDistance.cpp:30-49.
 // rn: an approximate reciprocal of valid (recip_nr; see ratio_f32), or 0.
-__device__ __forceinline__ float kimura_protein_of_p(float distance, const float *pam_dist,
-                                                     const double2 *tabq = nullptr);
+__device__ __forceinline__ float kimura_protein_of_p(float distance, const float *pam_dist);
 
 __device__ __forceinline__ float kimura_protein_distance(unsigned long long mism,
                                                          unsigned long long valid,
@@ -482,15 +459,14 @@ __device__ __forceinline__ float kimura_protein_distance(unsigned long long mism
 }
 
 // KimuraDistance.cpp:325-338 from the float p (-1 when valid is 0).  pam_dist:
-// the Dayhoff table's distances, (float)(PAM / 100.0) per entry; tabq: as jc_of_q.
-__device__ __forceinline__ float kimura_protein_of_p(float distance, const float *pam_dist,
-                                                     const double2 *tabq) {
+// the Dayhoff table's distances, (float)(PAM / 100.0) per entry.
+__device__ __forceinline__ float kimura_protein_of_p(float distance, const float *pam_dist) {
   const double dd = (double)distance;
   if (dd < 0.75) {
     if (dd > 0.0) {
       const double sq = (double)__fmul_rn(distance, distance);
       const double arg = __dsub_rn(__dsub_rn(1.0, dd), __dmul_rn(sq, 0.20));
-      const float fast = tabq ? neg_log_checked_tab(1.0, arg, tabq) : neg_log_checked(1.0, arg);
+      const float fast = neg_log_checked(1.0, arg);
       distance = fast == fast ? fast : neg_log_slow(1.0, arg);
     }
   } else {

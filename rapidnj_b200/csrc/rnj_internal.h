@@ -75,7 +75,10 @@ struct Packed {
   uint8_t *feat = nullptr;
   int Lk = 0;            // L rounded up to 256
   int nfb = 4;           // feature blocks of Lk columns: 4 (DNA), 1 + ranks (protein)
-  CUtensorMap fmap;      // 3-D map over (128, Np, nfb * Lk / 256), box (128, 128, 1), 128-byte swizzle
+  // 4-D maps over (128, Np, Lk / 256, nfb), 128-byte swizzle, of the fused kernel's
+  // operands: box (128, 128, 2, 1) and (128, 64, 2, 1).  (The one-CTA kernels' map
+  // is made where they are launched, encode_block_map.)
+  CUtensorMap fmap_a, fmap_b;
 };
 
 struct EpiParams {
@@ -102,7 +105,9 @@ struct EpiParams {
 // One alignment of a work list, as the persistent kernels read it from device
 // memory: its TMA map, output, scratch slots and transform parameters.
 struct alignas(128) AlnDesc {
-  CUtensorMap map;            // features (tensor-core kind) or planes (popcount kinds)
+  CUtensorMap map;            // planes (popcount kinds), or the one-CTA tensor-core kernels'
+                              // features (encode_block_map)
+  CUtensorMap map_a, map_b;   // features: Packed::fmap_a, fmap_b
   float *out;                 // n rows of ld floats (distances), or null in count mode
   uint32_t *counts;           // n*n*3 counts (count mode), or null
   unsigned long long ld;
@@ -115,17 +120,20 @@ struct alignas(128) AlnDesc {
                                // band: tile-order band height (single alignment), 0 = 12;
                                // wait_us: bound of the pipeline waits (0: 2 s)
   int stall, row0;             // stall, row0: as EpiParams
-  int stages, pad_;            // stages: the tensor-core ring depth of a work-list launch
-                               // (read from the first descriptor; 0: the launch's own)
+  int pad_[2];
   double jc_b;
 };
 static_assert(sizeof(AlnDesc) % 128 == 0, "descriptors of a work list share no 128-byte line");
 
-// A work item: alignment index and linear triangle-tile index within it.
+// A work item: alignment index and linear triangle-tile index within it.  For the
+// fused kernel (rnj_tcf.cu) an item is a pair of tile rows: tile is that of the
+// first row, and the second row's tile of the same column belongs to the item
+// when it lies in the triangle, unless kPairSingle is set.
 struct WorkItem {
   int aln;
   int tile;
 };
+constexpr int kPairSingle = (int)0x80000000;
 
 // Scratch of one distance call: the max slot, the error word and the per-tile
 // saturation flags (device), plus the split-K count buffer for long alignments.
@@ -211,6 +219,9 @@ cudaError_t launch_pack_features_prot(const uint8_t *d_chars, size_t ld, int n, 
 cudaError_t launch_pack_features_bits(const uint32_t *d_bits, const uint32_t *d_gaps, int bs_words,
                                       int n, int L, int Np, int Lk, uint8_t *F, cudaStream_t s);
 int encode_features_map(Packed &p);
+// The map of one 256-column K block of 128 rows (the kernels of rnj_tc.cu and the
+// live form) over p's features, into a descriptor.
+int encode_block_map(const Packed &p, CUtensorMap *map);
 // Batched popcount path (rnj_kernels.cu): persistent, atomic item counter.
 cudaError_t launch_count_batch(const AlnDesc *d_descs, const WorkItem *d_items, const int *d_nitems,
                                int *d_counter, int grid, int epi_mode, cudaStream_t s);
@@ -236,20 +247,25 @@ cudaError_t launch_tc_transform(const AlnDesc *d_descs, const WorkItem *d_items,
                                 const int *d_nitems, int nitems, int item0, int count,
                                 const uint64_t *packed, int grid, cudaStream_t s);
 // The fused form (rnj_tcf.cu): counts and the exact transform in one persistent
-// launch over work items [item0, min(n, item0 + count)) (d_items == nullptr: the
-// banded tiles of d_descs[0]; d_nitems == nullptr: n = nitems); distances
+// launch over work items [first, first + count), each a pair of tile rows of one
+// column tile (d_items == nullptr: the banded row pairs of d_descs[0], pair_items
+// of them, or with AlnDesc::full those of its row band); distances
 // straight into each alignment's output, with its max slot and saturation
 // flags.  Every alignment has at most kMaxFusedColumns columns.
 // variant: the transform of every item (fused_variant_for), or FUSED_ANY to
-// choose per item from its descriptor.  stages: the ring depth (0: the
-// default, 6; the tuner's tc_stages).
+// choose per item from its descriptor.  stages: the ring depth (0: the default, 6;
+// the tuner's tc_stages).
 enum FusedVariant {
   FUSED_K2P = 0, FUSED_JC = 1, FUSED_PROTEIN = 2, FUSED_GENERIC = 3, FUSED_FULL = 4, FUSED_ANY = 5
 };
 int fused_variant_for(int model, int type, int compat, int full);
-cudaError_t launch_tc_fused(const AlnDesc *d_descs, const WorkItem *d_items, const int *d_nitems,
-                            int nitems, int item0, int count, int grid, int variant,
-                            cudaStream_t s, int stages = 0);
+cudaError_t launch_tc_fused(const AlnDesc *d_descs, const WorkItem *d_items, int first, int count,
+                            int variant, cudaStream_t s, int stages = 0);
+// Row-pair work items for launch_tc_fused: of the columns tj >= r0 of tile rows
+// [r0, r1), and of the tiles [t0, t1) in row-major order of the triangle.
+long long pair_items(int nt);  // items of a whole triangle of nt tile rows
+void pair_items_of_band(int aln, int nt, int r0, int r1, std::vector<WorkItem> &out);
+void pair_items_of_range(int aln, int nt, long long t0, long long t1, std::vector<WorkItem> &out);
 // The ring depth launch_tc_fused runs with for a requested `stages`.
 int fused_ring_depth(int stages);
 

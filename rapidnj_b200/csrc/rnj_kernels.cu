@@ -787,8 +787,15 @@ __global__ void __launch_bounds__(256) fixup_batch_kernel(const AlnDesc *__restr
   for (int it = blockIdx.x; it < na + nb; it += gridDim.x) {
     const WorkItem w = it < na ? items_a[it] : items_b[it - na];
     const AlnDesc &d = descs[w.aln];
-    if (d.out == nullptr || d.tile_flags[w.tile] == 0) continue;
-    fixup_tile<4>(d, w.tile, __fmul_rn(__int_as_float(*d.max_bits), 2.0f), threadIdx.x, blockDim.x);
+    if (d.out == nullptr) continue;
+    const float m2 = __fmul_rn(__int_as_float(*d.max_bits), 2.0f);
+    const int tile = w.tile & ~kPairSingle;
+    if (d.tile_flags[tile] != 0) fixup_tile<4>(d, tile, m2, threadIdx.x, blockDim.x);
+    if (!is_tc_kind(d.kind) || (w.tile & kPairSingle)) continue;
+    int ti, tj;
+    tri_coords(tile, d.nt, ti, tj);  // a row pair: the second row's tile
+    const int second = tile + d.nt - ti - 1;
+    if (ti < tj && d.tile_flags[second] != 0) fixup_tile<4>(d, second, m2, threadIdx.x, blockDim.x);
   }
 }
 

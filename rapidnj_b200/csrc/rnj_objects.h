@@ -70,13 +70,15 @@ int ensure_packed(rnj_ctx *ctx, long long tiles);
 int run_tc_chunks(rnj_ctx *ctx, const rnj::AlnDesc *d_desc, const rnj::WorkItem *d_items,
                   long long nitems, uint64_t *packed, cudaStream_t s, int transform_ctas = 0,
                   int stages = 0);
-// Distances of work items [0, nitems) of one tensor-core alignment (descriptor
-// d_desc on the device; d_items == nullptr: its banded triangle): the fused
-// kernel (rnj_tcf.cu) when the alignment takes it (at most kMaxFusedColumns
-// columns, and the tuned choice), else run_tc_chunks (rnj_api.cu).
+// Whether a tensor-core alignment takes the fused kernel (rnj_tcf.cu): at most
+// kMaxFusedColumns columns, and the tuned choice; else run_tc_chunks.
+inline bool tc_fused_form(const rnj::Packed &p, const rnj::TuneParams &tp) {
+  return tp.tc_epilogue == 0 && p.L <= rnj::kMaxFusedColumns;
+}
+// Distances of the whole triangle of one tensor-core alignment (descriptor d_desc
+// on the device) by either form (rnj_api.cu).
 int run_tc_distances(rnj_ctx *ctx, const rnj::Packed &p, const rnj::EpiParams &ep,
-                     const rnj::AlnDesc *d_desc, const rnj::WorkItem *d_items, long long nitems,
-                     cudaStream_t s, const rnj::TuneParams &tp);
+                     const rnj::AlnDesc *d_desc, cudaStream_t s, const rnj::TuneParams &tp);
 
 struct rnj_aln {
   rnj_ctx *ctx = nullptr;

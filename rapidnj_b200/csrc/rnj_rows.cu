@@ -159,11 +159,12 @@ extern "C" int rnj_distance_rows(rnj_ctx *ctx, rnj_aln *aln, int model, int band
     if (tc) {
       AlnDesc d = desc_for(p, eb);
       d.full = 1;
+      d.band = t1 - t0;  // the band's tile rows, taken in pairs
+      const int pairs = (t1 - t0 + 1) / 2 * nt;
       RNJ_TRY(cudaMemcpyAsync(buf.d_desc[b], &d, sizeof(d), cudaMemcpyHostToDevice, ctx->stream),
               "band descriptor upload");
-      RNJ_TRY(launch_tc_fused(buf.d_desc[b], nullptr, nullptr, (int)all_tiles, (int)tile0,
-                              (int)btiles, (int)std::min<long long>(btiles, ctx->num_sms),
-                              FUSED_FULL, ctx->stream, tp.tc_stages),
+      RNJ_TRY(launch_tc_fused(buf.d_desc[b], nullptr, 0, pairs, FUSED_FULL, ctx->stream,
+                              tp.tc_stages),
               "fused tensor-core kernel (row band)");
     } else {
       const int ckind = (p.kind == KIND_DNA && model == RNJ_JC) ? KIND_MISM2 : p.kind;

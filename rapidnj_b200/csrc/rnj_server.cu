@@ -381,6 +381,9 @@ void prepare_all(rnj_server *s, const std::vector<Request *> &reqs) {
       ep.err = s->live.err;
       s->h_descs[slot] = desc_for(p, ep);
       s->h_done[slot] = make_int2(0, 0);
+      if (encode_block_map(p, &s->h_descs[slot].map) != RNJ_OK) e = cudaErrorInvalidValue;
+    }
+    if (e == cudaSuccess) {
       e = cudaMemcpyAsync(s->d_descs + slot, s->h_descs + slot, sizeof(AlnDesc),
                           cudaMemcpyHostToDevice, ctx->stream);
     }

@@ -32,6 +32,9 @@ struct rnj_shard {
   int model = RNJ_KIMURA;
   int full = 0;
   long long t0 = 0, t1 = 0, ntiles = 0;
+  TuneParams tp;           // the bucket's choices when the shard was made
+  bool fused = false;      // items are row pairs for the fused kernel
+  long long nitems = 0;
   float *out = nullptr;
   size_t ld = 0;
   bool owns_out = false;
@@ -140,7 +143,13 @@ int rnj_shard_create(rnj_ctx *ctx, rnj_aln *aln, int model, int shard, int nshar
   s->owns_out = (d_out == nullptr);
   s->ld = d_out ? ld : (size_t)std::max(4, (p.n + 3) / 4 * 4);
   s->out = d_out;
-  const long long nitems = t1 - t0;
+  s->tp = tune_lookup(p.n, p.L, p.type, p.flags);
+  s->fused = is_tc_kind(p.kind) && tc_fused_form(p, s->tp);
+  std::vector<WorkItem> items;
+  if (s->fused) pair_items_of_range(0, tiles_of(p.n), t0, t1, items);
+  else
+    for (long long t = t0; t < t1; ++t) items.push_back(WorkItem{0, (int)t});
+  const long long nitems = s->nitems = (long long)items.size();
   cudaStream_t st = ctx->stream;
   cudaError_t e = cudaSuccess;
   if (!d_out) e = cudaMallocAsync((void **)&s->out, s->ld * p.n * sizeof(float), st);
@@ -153,8 +162,6 @@ int rnj_shard_create(rnj_ctx *ctx, rnj_aln *aln, int model, int shard, int nshar
     free_shard(s);
     return cuda_error(e, "shard allocation");
   }
-  std::vector<WorkItem> items((size_t)nitems);
-  for (long long k = 0; k < nitems; ++k) items[(size_t)k] = WorkItem{0, (int)(t0 + k)};
   const int ints[4] = {(int)nitems, 0, 0, 0};
   EpiParams ep = epi_params_for(p, model);
   ep.out = s->out;
@@ -162,7 +169,11 @@ int rnj_shard_create(rnj_ctx *ctx, rnj_aln *aln, int model, int shard, int nshar
   ep.max_bits = s->d_words;
   ep.err = s->d_words + 1;
   ep.tile_flags = s->d_words + 2;
-  const AlnDesc d = desc_for(p, ep);
+  AlnDesc d = desc_for(p, ep);
+  if (is_tc_kind(p.kind) && !s->fused && (rc = encode_block_map(p, &d.map)) != RNJ_OK) {
+    free_shard(s);
+    return rc;
+  }
   // Pageable sources: each copy has consumed its source when the call returns.
   e = cudaMemcpyAsync(s->d_desc, &d, sizeof(d), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && nitems)
@@ -183,17 +194,27 @@ int rnj_shard_run(rnj_shard *s, float *local_max) {
   DeviceGuard g(ctx->device);
   cudaStream_t st = ctx->stream;
   const Packed &p = s->aln->p;
-  const long long nitems = s->t1 - s->t0;
+  const long long nitems = s->nitems;
   RNJ_CUDA(cudaMemsetAsync(s->d_words, 0, (s->ntiles + 2) * sizeof(int), st), "shard scratch clear");
   RNJ_CUDA(cudaMemsetAsync(s->d_ints + 1, 0, sizeof(int), st), "shard counter clear");
   if (p.n == 1 && nitems > 0)
     RNJ_CUDA(cudaMemsetAsync(s->out, 0, sizeof(float), st), "diagonal");
   if (nitems > 0) {
     const int grid = (int)std::min<long long>(nitems, ctx->num_sms);
-    if (is_tc_kind(p.kind)) {
+    if (s->fused) {
+      const EpiParams ep = epi_params_for(p, s->model);
+      ctx_mark(ctx, 1, 0);
+      RNJ_CUDA(launch_tc_fused(s->d_desc, s->d_items, 0, (int)nitems,
+                               fused_variant_for(ep.model, ep.type, ep.compat_wrap, 0), st,
+                               s->tp.tc_stages),
+               "fused tensor-core kernel");
+      ctx_mark(ctx, 1, 1);
+    } else if (is_tc_kind(p.kind)) {
       // Marks stage 1 around the counting kernels.
-      const int rc = run_tc_distances(ctx, p, epi_params_for(p, s->model), s->d_desc, s->d_items,
-                                      nitems, st, tune_lookup(p.n, p.L, p.type, p.flags));
+      int rc = ensure_packed(ctx, std::min<long long>(nitems, kTcChunkTiles));
+      if (rc == RNJ_OK)
+        rc = run_tc_chunks(ctx, s->d_desc, s->d_items, nitems, ctx->d_packed, st,
+                           s->tp.transform_ctas, s->tp.tc_stages);
       if (rc != RNJ_OK) return rc;
     } else {
       ctx_mark(ctx, 1, 0);
@@ -211,7 +232,7 @@ int rnj_shard_finish(rnj_shard *s, float global_max) {
   rnj_ctx *ctx = s->ctx;
   DeviceGuard g(ctx->device);
   cudaStream_t st = ctx->stream;
-  const long long nitems = s->t1 - s->t0;
+  const long long nitems = s->nitems;
   if (nitems == 0) return RNJ_OK;
   memcpy(ctx->h_max, &global_max, sizeof(float));
   RNJ_CUDA(cudaMemcpyAsync(s->d_words, ctx->h_max, sizeof(int), cudaMemcpyHostToDevice, st),

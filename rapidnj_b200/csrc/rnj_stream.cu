@@ -214,13 +214,14 @@ int distance_host_streamed(rnj_ctx *ctx, const char *chars, int n, int L, size_t
   for (int k = 0; k < nbands; ++k) {
     const int t0 = bounds[k + 1], t1 = bounds[k];
     band_off[k] = (long long)items.size();
+    if (fused) {
+      pair_items_of_band(0, nt, t0, t1, items);
+      continue;
+    }
     for (int tj = t0; tj < nt; ++tj)
-      for (int ti = t0; ti < t1 && ti <= tj; ++ti) {
-        WorkItem w;
-        w.aln = 0;
-        w.tile = (int)((long long)ti * nt - (long long)ti * (ti - 1) / 2 + (tj - ti));
-        items.push_back(w);
-      }
+      for (int ti = t0; ti < t1 && ti <= tj; ++ti)
+        items.push_back(
+            WorkItem{0, (int)((long long)ti * nt - (long long)ti * (ti - 1) / 2 + (tj - ti))});
   }
   band_off[nbands] = (long long)items.size();
 
@@ -269,6 +270,7 @@ int distance_host_streamed(rnj_ctx *ctx, const char *chars, int n, int L, size_t
   ep.out = buf.out;
   ep.ld = (size_t)n;
   AlnDesc desc = desc_for(p, ep);
+  if (!fused && (rc = encode_block_map(p, &desc.map)) != RNJ_OK) return rc;
   RNJ_TRY(cudaMemcpyAsync(ctx->d_desc, &desc, sizeof(desc), cudaMemcpyHostToDevice, ctx->stream),
           "descriptor upload");
 
@@ -314,8 +316,7 @@ int distance_host_streamed(rnj_ctx *ctx, const char *chars, int n, int L, size_t
             "feature pack kernel");
     const long long i0 = band_off[k], cnt = band_off[k + 1] - band_off[k];
     if (fused) {
-      RNJ_TRY(launch_tc_fused(ctx->d_desc, buf.items, nullptr, (int)items.size(), (int)i0,
-                              (int)cnt, (int)std::min<long long>(cnt, ctx->num_sms),
+      RNJ_TRY(launch_tc_fused(ctx->d_desc, buf.items, (int)i0, (int)cnt,
                               fused_variant_for(ep.model, ep.type, ep.compat_wrap, 0),
                               ctx->stream, tp.tc_stages),
               "fused tensor-core kernel");
@@ -350,9 +351,11 @@ int distance_host_streamed(rnj_ctx *ctx, const char *chars, int n, int L, size_t
           "flag copy");
   RNJ_TRY(cudaStreamSynchronize(ctx->stream), "first band sync");
   {
+    // (the first band: tile rows bounds[1] .. nt - 1, the end of the row-major order)
+    const long long r = bounds[1], first = r * nt - r * (r - 1) / 2;
     long long sat = 0;
-    for (long long it = band_off[0]; it < band_off[1]; ++it) sat += ctx->h_words[2 + items[it].tile] != 0;
-    deferred = sat * 4 > band_off[1] - band_off[0];
+    for (long long t = first; t < ntiles; ++t) sat += ctx->h_words[2 + t] != 0;
+    deferred = sat * 4 > ntiles - first;
   }
   for (int k = 1; k < nbands; ++k) {
     rc = run_band(k);

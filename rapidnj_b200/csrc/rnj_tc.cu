@@ -460,13 +460,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int half = (warp - 2) >> 2;
     const int row = 32 * q + lane;
     uint32_t titer = 0;
+    TileWalk walk(descs, items);
     for (int it = item0 + blockIdx.x; it < nitems; it += gridDim.x, ++titer) {
-      const WorkItem w = item_at(descs, items, it);
-      const AlnDesc &d = descs[w.aln];
-      int ti, tj;
-      item_tile(d, w.tile, ti, tj);
+      const TileAt at = walk.at(it);
+      const AlnDesc &d = descs[at.aln];
+      const int ti = at.ti, tj = at.tj;
       if ((stall && titer == 0 && !tc_wait(sh.never_bar, 0, sh.abort_flag, limit)) ||
-          !tc_wait(sh.acc_full, titer & 1, sh.abort_flag, limit)) {
+          !tc_wait(&sh.acc_full[1], titer & 1, sh.abort_flag, limit)) {
         *sh.abort_flag = 1;
         break;
       }
@@ -488,7 +488,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         tmem_ld_wait();
         if (cc == 1) {
           tc_fence_before();
-          mbar_arrive(sh.tmem_empty);
+          mbar_arrive(&sh.tmem_empty[0]);
+          mbar_arrive(&sh.tmem_empty[1]);
         }
         const int jb = tj * kTile + cbase;
 #pragma unroll
@@ -547,11 +548,11 @@ __global__ void __launch_bounds__(kTransformThreads, kTransformCtasPerSm)
   const int nitems = (int)min((long long)(nitems_ptr ? *nitems_ptr : nitems_direct),
                               (long long)item0 + count);
   const int rblk = 32 * (warp & 3), chalf = 64 * (warp >> 2);
+  TileWalk walk(descs, items);
   for (int it = item0 + blockIdx.x; it < nitems; it += gridDim.x) {
-    const WorkItem w = item_at(descs, items, it);
-    const AlnDesc &d = descs[w.aln];
-    int ti, tj;
-    item_tile(d, w.tile, ti, tj);
+    const TileAt at = walk.at(it);
+    const AlnDesc &d = descs[at.aln];
+    const int ti = at.ti, tj = at.tj;
     EpiParams ep;
     ep.n = d.n;
     ep.L = d.L;
@@ -610,7 +611,7 @@ __global__ void __launch_bounds__(kTransformThreads, kTransformCtasPerSm)
     const bool any_sat = __any_sync(0xffffffffu, sat);
     if (lane == 0) {
       if (tmax > 0.0f) atomicMax(d.max_bits, __float_as_int(tmax));
-      if (any_sat) d.tile_flags[w.tile] = 1;
+      if (any_sat) d.tile_flags[at.tile] = 1;
     }
   }
 }

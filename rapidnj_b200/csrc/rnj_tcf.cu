@@ -2,34 +2,51 @@
 // tensor cores and the exact transform in the same CTA, straight from tensor
 // memory to the distance matrix.
 //
-// The counting pipeline is the one of rnj_tcgen05.cuh (warp 16 TMA producer,
-// warp 17 MMA issuer, three f32 accumulators V, R, T of 128 x 128 in tensor
-// memory, a six-stage ring).  Sixteen epilogue warps (0 .. 15, with 112
-// registers each after a setmaxnreg split) replace the packed-count round trip
-// of the two-kernel form (8 bytes per pair written and read again, then a
-// separate transform launch):
+// The counting pipeline is the pair form of rnj_tcgen05.cuh: two CTAs of a
+// cluster on one 256 x 128 tile (in each, warp 16 is the TMA producer; the
+// leader's warp 17 issues the MMAs of both), three f32 accumulators V, R, T of
+// 128 x 128 in each CTA's tensor memory, a ring of four stages of two K blocks.
+// The live form of the server (below) claims single tiles and runs the one-CTA
+// pipeline.  Sixteen epilogue warps (0 .. 15, with 112 registers each after a
+// setmaxnreg split) replace the packed-count round trip of the two-kernel form
+// (8 bytes per pair written and read again, then a separate transform launch):
 //   * warp w reads tensor-memory lane quarter w % 4 (32 tile rows, lane = row)
-//     and columns 32 (w / 4) .. + 31 of the three accumulators, 16
-//     columns at a time, converts them to integer counts (16 bits each: the
-//     fused form takes alignments of at most 65535 columns) and hands tensor
-//     memory back to the MMA warp at once;
-//   * it then computes the 32 distances of each lane from registers, sixteen
-//     pairs at a time (K2P: k2p_decide16, with the logarithm table copied to
-//     shared memory; the quotients by the valid count from its Newton-Raphson
-//     reciprocal, the same floats as the reference's divisions, ratio_f32)
-//     while the tensor cores already count the next tile;
+//     and columns 32 (w / 4) .. + 31 of the three accumulators: V as soon as it
+//     is complete, packed to 16 bits (the fused form takes alignments of at most
+//     65535 columns), then R and T sixteen columns at a time at the tile's end,
+//     each part handed back to the MMA warp once read (rnj_tcgen05.cuh);
+//   * it computes the distances of each lane from the f32 sums as they are,
+//     eight pairs at a time without branches: exact sums and differences, the
+//     quotients by the valid count in float (the same floats as the reference's
+//     divisions, quotient_of), a and b in double, the logarithm from a
+//     table in shared memory (neg_quarter_ln) and the rounding check
+//     (RoundCheck), while the tensor cores already count the next tile;
 //   * stores: the mirror entries out[j][i] as coalesced 128-byte row segments
-//     (lanes are consecutive i), the tile entries out[i][j .. j + 3] as 16-byte
-//     vectors, the diagonal as 0; the tile's maximum goes to the alignment's
-//     max slot (atomicMax on the float bits) and a saturated pair (-1) sets
-//     the tile's flag for the fix-up kernel.  With AlnDesc::full the work items
-//     are full-square tiles of a band of rows (out-of-core delivery): every
-//     ordered pair is stored in its row of the band buffer, no mirror.
+//     (lanes are consecutive i), the tile entries out[i][j .. j + 7] as one
+//     32-byte vector per lane, a full sector (two 16-byte ones, or through a
+//     per-warp transpose in shared memory, where the row stride or the base
+//     does not allow it), the diagonal as 0; the tile's maximum goes to the
+//     alignment's max slot (atomicMax on the float bits) and a saturated pair
+//     (-1) sets the tile's flag for the fix-up kernel.  With AlnDesc::full the
+//     work items are full-square tiles of a band of rows (out-of-core delivery):
+//     every ordered pair is stored in its row of the band buffer, no mirror.
 // The transform's instructions overlap the MMAs of the next tile instead of
 // following them in a second kernel.
+//
+// What bounds it.  Long alignments: the MMAs of a pair, 326 cycles per 256
+// columns with operands at rest, 343 with loads, 436 with the epilogue at work
+// (10,000 x 10,000 DNA step 1.00 -> 0.955 ms; the chip is at its 1,000 W limit
+// there, 1.76 GHz).  Short ones: the epilogue, 18,000 cycles a tile for the K2P
+// transform, 73 warp instructions per 32 pairs (168 before: 50,000 x 1,000 step
+// 7.58 -> 5.79 ms), no pipe above a third of its rate; of what it does, the
+// stores cost 15 %, the table reads 9 %, each double operation about 1.7 %.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
+#include <atomic>
+#include <vector>
 
 #include "rnj_device.cuh"
 #include "rnj_epilogue.cuh"
@@ -50,15 +67,48 @@ constexpr int kTcfProducerWarp = 16, kTcfMmaWarp = 17;
 constexpr int kTcfRegsLow = 32, kTcfRegsHigh = 112, kTcfRegsLaunch = 96;
 static_assert(128 * kTcfRegsLow + 512 * kTcfRegsHigh <= kTcfThreads * kTcfRegsLaunch,
               "the register split fits the launch's registers");
-// A ring of up to six stages (a seventh stage's 32 KB would leave no room; six
-// is the default, the tuner may choose fewer) and the logarithm table
-// (128 x {-ln F / 4, -1 / (4 F)}, the scaled table of neg_quarter_ln_table_k)
-// after the barrier block.
+// A ring of up to six 256-column K blocks of two operand tiles, 32 KB each (the
+// default; the tuner may choose fewer), which hold 2/3 as many stages of a CTA of
+// a pair, and, after the barrier block, the
+// logarithm table (128 entries of two doubles, eight copies), the Dayhoff
+// distances and the transpose buffers of the epilogue warps (32 rows of eight
+// columns).
 constexpr int kTcfStages = 6;
-constexpr size_t kTcfTableBytes = 128 * 2 * sizeof(double);
-constexpr size_t kTcfSmemBytes = tc_smem_bytes(kTcfStages, kTcfTableBytes);
+constexpr size_t kTcfTableBytes = kLnIntervals * kLnCopies * 2 * sizeof(double);
+constexpr size_t kTcfPamBytes = 768;
+constexpr size_t kTcfWarpStage = 32 * 8 * sizeof(float);
+constexpr size_t kTcfExtra = kTcfTableBytes + kTcfPamBytes + kTcfEpiWarps * kTcfWarpStage;
+constexpr size_t kTcfSmemBytes = tc_smem_bytes(kPairStages, kTcfExtra, kPairStageBytes);
 static_assert(kTcfSmemBytes <= 232448, "fits the shared memory of one CTA");
-constexpr int kTcfGroup = 4;                         // pairs per transform group
+static_assert(sizeof(c_pam.dist) <= kTcfPamBytes, "the Dayhoff distances fit their slot");
+
+// Stages of the pair form in the ring of a requested depth (0: the default).
+__host__ __device__ constexpr int pair_stages(int depth) {
+  const int st = tc_ring_depth(depth, kTcfStages, kTcfStages) * 2 / 3;
+  return st < kTcMinStages ? kTcMinStages : st;
+}
+static_assert(pair_stages(0) == kPairStages, "the deepest ring");
+
+// The tables (ln: this lane's copy) and this warp's transpose buffer.
+struct TcfTables {
+  const double2 *ln;
+  const float *pam;
+  float *stage;
+};
+
+// The tables into shared memory (every thread of the block; published by
+// tc_setup's block barriers).
+__device__ __forceinline__ TcfTables tcf_tables(const TcShared &sh) {
+  uint8_t *const x = tc_extra(sh);
+  double2 *const ln = reinterpret_cast<double2 *>(x);
+  float *const pam = reinterpret_cast<float *>(x + kTcfTableBytes);
+  for (int e = threadIdx.x; e < kLnIntervals * kLnCopies; e += kTcfThreads)
+    ln[e] = make_double2(__ldg(&c_log_tab_q[e / kLnCopies][0]), __ldg(&c_log_tab_q[e / kLnCopies][1]));
+  if (threadIdx.x < 181) pam[threadIdx.x] = __ldg(c_pam.dist + threadIdx.x);
+  return {ln + threadIdx.x % kLnCopies, pam,
+          reinterpret_cast<float *>(x + kTcfTableBytes + kTcfPamBytes +
+                                    (threadIdx.x >> 5) % kTcfEpiWarps * kTcfWarpStage)};
+}
 
 // Transform variants of the fused epilogue, one loop each so that only the
 // model's own parameters stay in registers (kFusedK2p .. kFusedAny are the
@@ -68,379 +118,514 @@ enum {
   kFusedGeneric = FUSED_GENERIC, kFusedFull = FUSED_FULL, kFusedAny = FUSED_ANY
 };
 
+// Integer counts from the f32 sums (exact integers): DNA transitions P = (V + R
+// - T) / 4 and transversions Q = (V - R) / 2, protein mismatches V - M and 0.
+__device__ __forceinline__ void counts_of(bool prot, float fv, float fr, float ft, uint32_t &c0,
+                                          uint32_t &c1, uint32_t &vv) {
+  const float d = __fsub_rn(fv, fr);
+  vv = __float2uint_rn(fv);
+  c0 = prot ? __float2uint_rn(d) : __float2uint_rn(0.25f * __fsub_rn(__fadd_rn(fv, fr), ft));
+  c1 = prot ? 0u : __float2uint_rn(0.5f * d);
+}
+
+// The transform of one pair from its counts, any model and flags.
+__device__ __forceinline__ float generic_pair(const AlnDesc &d, float fv, float fr, float ft) {
+  EpiParams ep;
+  ep.n = d.n;
+  ep.L = d.L;
+  ep.model = d.model;
+  ep.type = d.type;
+  ep.compat_wrap = d.compat;
+  ep.jc_b = d.jc_b;
+  uint32_t c0, c1, vv;
+  counts_of(d.kind == KIND_PROT_TC, fv, fr, ft, c0, c1, vv);
+  return pair_distance(ep, c0, c1, vv, true);
+}
+
+// Out of line: the rare pairs that the rounding check leaves undecided.
+template <int M, bool kProt>
+static __device__ __noinline__ float fused_undecided(float fv, float fr, float ft) {
+  uint32_t c0, c1, vv;
+  counts_of(kProt, fv, fr, ft, c0, c1, vv);
+  if (M == kFusedK2p) return k2p_distance(c0, c1, vv);
+  if (M == kFusedProtein) return kimura_protein_distance(c0, vv, c_pam.dist);
+  return jc_distance((unsigned long long)c0 + c1, vv, kProt ? 0.95 : 0.75);
+}
+
+// A pair of a model's transform, without branches: the distance (-1 when
+// saturated), and through `slow` whether the rounding check could not decide it
+// (fused_undecided then gives the value).  m (margin, below) bounds the
+// difference between the double computed here and the reference's, in units
+// of 2^-53 of it; the terms besides neg_quarter_ln's 2^-42 = 2^11 units:
+//   K2P (KimuraDistance.cpp:339-349)   a, b are the reference's doubles; a a b is
+//     within 2^-52 (relative) of a^2 b, so its logarithm is off by 2^-52 at most
+//     and |ln(a^2 b)| = 4 D >= 4 (1 - 2^-23) / n: n / 2 units; the reference's own
+//     two logarithms and subtraction: 3 units.  m = 4096 + L.
+//   JC (JCdistance.cpp:171-183)        1 - q is the reference's double; a few
+//     units.  m = 4096.
+//   protein Kimura (KimuraDistance.cpp:322-338)   1 - p - p^2 / 5 has one rounding
+//     instead of two: 2^-53 + 2^-56 absolute on an argument of at least 0.137,
+//     relative to its logarithm at most 2 n units.  m = 4096 + 2 L.
+// Undecided pairs: 2 m / 2^29 of all (about 2e-5 at L = 1000).
 template <int M>
-__device__ __forceinline__ float fused_pair(const AlnDesc &d, uint32_t ts, uint32_t tv,
-                                            uint32_t vv, double jc_inv_b = 0.0,
-                                            const double2 *tab = nullptr) {
-  if constexpr (M == kFusedJc || M == kFusedProtein) {
-    // the float quotient by the valid count in float arithmetic (quotient16:
-    // counts below 2^16 here, the count of differences at most the valid count)
-    const float fv = __fsub_rn(__uint_as_float(0x4B000000u | (vv ? vv : 1u)), 8388608.0f);
-    const float y = recip16(fv);
-    if constexpr (M == kFusedJc)  // jc_inv_b: 1 / d.jc_b, correctly rounded
-      return jc_of_q(div_by_b(vv ? (double)quotient16(ts + tv, fv, y) : 0.0, d.jc_b, jc_inv_b),
-                     d.jc_b, tab);
-    else
-      return kimura_protein_of_p(vv ? quotient16(ts, fv, y) : -1.0f, c_pam.dist, tab);
+__device__ __forceinline__ uint32_t margin(int L) {
+  return M == kFusedK2p ? 4096u + (uint32_t)L : (M == kFusedProtein ? 4096u + 2u * (uint32_t)L : 4096u);
+}
+
+// The double part of a pair's transform, from its quotients: K2P qa = 4 P / n, qb =
+// 2 Q / n; JC and protein qa = p.
+template <int M, bool kProt>
+__device__ __forceinline__ float fused_value(float qa, float qb, double inv_b, const RoundCheck &rc,
+                                             const TcfTables &tab, bool &slow) {
+  uint32_t t2;
+  if constexpr (M == kFusedK2p) {
+    const double ts4 = (double)qa, tv2 = (double)qb;
+    // 1 - 2 ts and then - tv, each the reference's one rounding (the products
+    // by a power of two are exact)
+    const double a = __fma_rn(-0.5, tv2, __fma_rn(-0.5, ts4, 1.0));
+    const double b = __dsub_rn(1.0, tv2);
+    const double dd = neg_quarter_ln(__dmul_rn(__dmul_rn(a, a), b), tab.ln, t2);
+    // a or b zero, negative or NaN (no valid site): bit 30 or 31 of one of
+    // these words.  Their float is positive exactly when they are: a nonzero
+    // one is a multiple of 2^-41.
+    const uint32_t w = t2 | (uint32_t)__double2hiint(a) | (uint32_t)__double2hiint(b);
+    slow = rc.undecided(dd);  // (no harm for a saturated pair)
+    return w < 0x40000000u ? __double2float_rn(dd) : -1.0f;
+  } else if constexpr (M == kFusedJc) {
+    constexpr double b = kProt ? 0.95 : 0.75;
+    const double arg = __dsub_rn(1.0, div_by_b((double)qa, b, inv_b));
+    const double dd = __dmul_rn(4.0 * b, neg_quarter_ln(arg, tab.ln, t2));
+    // q = fl(p / b) >= 1 exactly when p is at least b: 3/4, or the float above 19/20
+    const bool sat = qa >= (kProt ? 0.95000005f : 0.75f);
+    slow = rc.undecided(dd) && !sat;
+    return sat ? -1.0f : __double2float_rn(dd);
   } else {
-    EpiParams ep;
-    ep.n = d.n;
-    ep.L = d.L;
-    ep.model = d.model;
-    ep.type = d.type;
-    ep.compat_wrap = d.compat;
-    ep.jc_b = d.jc_b;
-    return pair_distance(ep, ts, tv, vv, true);
+    const float p = qa;
+    const double dp = (double)p;
+    const double arg = __fma_rn((double)__fmul_rn(p, p), -0.20, __dsub_rn(1.0, dp));
+    const double dd = neg_quarter_ln(arg, tab.ln, t2);
+    slow = rc.undecided(dd) && p < 0.75f;
+    // the float of 4 dd; the magnitude, for p = 0 gives +0
+    float x = fabsf(4.0f * __double2float_rn(dd));
+    if (p >= 0.75f) {
+      // the Dayhoff band: entry floor(1000 p - 750) in the reference's doubles,
+      // the floor by an addition of 2^52 rounded towards zero
+      const double t = __dsub_rn(__dmul_rn(dp, 1000.0), 750.0);
+      const int idx = __double2loint(__dadd_rz(t, 4503599627370496.0));
+      // (double)p > 0.930 iff p >= 0.93f
+      x = p >= 0.93f ? 10.0f : tab.pam[min((uint32_t)idx, 180u)];
+    }
+    return x;
   }
 }
 
-// k2p_distance out of line: the rare pairs whose one-logarithm value the
-// rounding check cannot decide.
-static __device__ __noinline__ float k2p_undecided(uint32_t P, uint32_t Q, uint32_t n) {
-  return k2p_distance(P, Q, n);
+// Two pairs: v23 = 2^23 + valid counts, fr and ft the other sums.
+template <int M, bool kProt>
+__device__ __forceinline__ void fused_pair2(f32x2 v23, f32x2 fr, f32x2 ft, double inv_b,
+                                            const RoundCheck &rc, const TcfTables &tab, float &x0,
+                                            float &x1, bool &slow0, bool &slow1) {
+  const f32x2 neg = pack2(-1.0f, -1.0f), bias = pack2(8388608.0f, 8388608.0f);
+  f32x2 fv = add2(v23, pack2(-8388608.0f, -8388608.0f)), nv = fma2(v23, neg, bias);
+  float qa0, qa1, qb0 = 0.0f, qb1 = 0.0f;
+  if constexpr (M == kFusedK2p) {
+    const f32x2 y = recip16_2(fv, nv);  // not finite for fv = 0: NaNs, -1 in the end
+    unpack2(quotient_of_2(fma2(ft, neg, add2(fv, fr)), nv, y), qa0, qa1);  // 4 P / n
+    unpack2(quotient_of_2(fma2(fr, neg, fv), nv, y), qb0, qb1);            // 2 Q / n
+    x0 = fused_value<M, kProt>(qa0, qb0, inv_b, rc, tab, slow0);
+    x1 = fused_value<M, kProt>(qa1, qb1, inv_b, rc, tab, slow1);
+  } else {
+    f32x2 num;  // mismatches V - M, or P + Q = (3 V - R - T) / 4
+    if (kProt) num = fma2(fr, neg, fv);
+    else
+      num = mul2(pack2(0.25f, 0.25f), fma2(pack2(3.0f, 3.0f), fv, mul2(neg, add2(fr, ft))));
+    float v0, v1;  // no valid site: p = 0 (JC), -1 (protein Kimura, below)
+    unpack2(fv, v0, v1);
+    fv = pack2(fmaxf(v0, 1.0f), fmaxf(v1, 1.0f));
+    nv = mul2(fv, neg);
+    unpack2(quotient_of_2(num, nv, recip16_2(fv, nv)), qa0, qa1);
+    x0 = fused_value<M, kProt>(qa0, qb0, inv_b, rc, tab, slow0);
+    x1 = fused_value<M, kProt>(qa1, qb1, inv_b, rc, tab, slow1);
+    if constexpr (M == kFusedProtein) {
+      x0 = v0 < 0.5f ? -1.0f : x0;
+      x1 = v1 < 0.5f ? -1.0f : x1;
+    }
+  }
 }
 
-// The 32 distances of row i, columns jb .. jb + 31 (counts pq / pv, see the
-// epilogue): the mirror entries out[j][i], the row entries out[i][j] for j >= i
-// (0 on the diagonal), the running maximum and whether a pair saturated.
-// tab: the logarithm table in shared memory, scaled by -1/4.
-template <int M>
-__device__ __forceinline__ void fused_rows(const AlnDesc &d, int i, int jb, uint32_t (&pq)[32],
-                                           uint32_t (&pv)[16], float &tmax, bool &sat,
-                                           const double2 *tab) {
-  const int n = d.n;
-  float *const out = d.out;
-  const size_t ld = d.ld;
-  const bool vec = ((ld & 3) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
-  float *const orow = out + (size_t)i * ld;  // dereferenced only for i < n
-  const double jc_inv_b = M == kFusedJc ? __ddiv_rn(1.0, d.jc_b) : 0.0;  // once per row
-#pragma unroll 1
-  for (int g = 0; g < 32 / kTcfGroup; ++g) {
-    const int j0 = jb + kTcfGroup * g;
-    float x[kTcfGroup];
-    {
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
+// How row entries are stored: 32 or 16 bytes a lane, or through the transpose
+// buffer (a row stride or base that no vector fits).
+enum RowStore { kRowVec8, kRowVec4, kRowStaged };
+
+__device__ __forceinline__ void store8(float *p, const float (&x)[8]) {
+  asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(x[0]),
+               "f"(x[1]), "f"(x[2]), "f"(x[3]), "f"(x[4]), "f"(x[5]), "f"(x[6]), "f"(x[7])
+               : "memory");
+}
+
+// The distances of row i (lane = row; rows i - lane .. + 31 of the warp), eight
+// columns j0 .. j0 + 7: the mirror entries out[j][i], the row entries out[i][j]
+// for j >= i (0 on the diagonal).  interior: every pair counts, no masks.
+__device__ __forceinline__ void store_group(float *out, size_t ld, int n, int i, int j0,
+                                            bool interior, RowStore how, const float (&x)[8],
+                                            float *stage) {
+  float *mp = out + (size_t)j0 * ld + i;
+  float *const rp = out + (size_t)i * ld + j0;  // dereferenced only for i < n
+  if (interior) {
+    // (interior tiles have ld < 2^32: one 32 x 32-bit multiply-add per address)
 #pragma unroll
-      for (int k = 0; k < kTcfGroup; ++k) {
-        const int j = j0 + k;
-        x[k] = 0.0f;
-        if (i < j && j < n) {
-          const uint32_t vv = (pv[k >> 1] >> (16 * (k & 1))) & 0xFFFFu;
-          x[k] = fused_pair<M>(d, pq[k] & 0xFFFFu, pq[k] >> 16, vv, jc_inv_b, tab);
-          tmax = fmaxf(tmax, x[k]);
-          sat |= (x[k] == -1.0f);
-          __stcs(out + (size_t)j * ld + i, x[k]);  // mirror: consecutive i across lanes
-        }
+    for (int k = 0; k < 8; ++k) __stcs(mp + (size_t)(uint32_t)ld * (uint32_t)k, x[k]);
+    if (how == kRowVec8) {
+      store8(rp, x);
+    } else if (how == kRowVec4) {
+      __stcs(reinterpret_cast<float4 *>(rp), make_float4(x[0], x[1], x[2], x[3]));
+      __stcs(reinterpret_cast<float4 *>(rp + 4), make_float4(x[4], x[5], x[6], x[7]));
+    } else {
+      // eight lanes per row: 32-byte runs instead of a 4-byte store per sector
+      // (word k of a row sits at k ^ (row / 4 % 8): neither the writes, a column
+      // at a time, nor the reads, four rows at a time, meet on a bank)
+      const int lane = threadIdx.x & 31;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) stage[lane * 8 + (k ^ (lane >> 2))] = x[k];
+      __syncwarp();
+      float *q = out + (size_t)(i - lane + (lane >> 3)) * ld + j0 + (lane & 7);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        __stcs(q, stage[(4 * k + (lane >> 3)) * 8 + ((lane & 7) ^ k)]);
+        q += 4 * ld;
       }
+      __syncwarp();
     }
-    // Row i, columns j0 .. j0 + 7 (j >= i; the diagonal is 0).
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int j = j0 + k;
+      if (i < j && j < n) __stcs(mp, x[k]);
+      mp += ld;
+    }
     if (i < n) {
 #pragma unroll
-      for (int h = 0; h < kTcfGroup / 4; ++h) {
-        const int jj = j0 + 4 * h;
-        if (vec && i < jj && jj + 3 < n) {
-          __stcs(reinterpret_cast<float4 *>(orow + jj),
-                 make_float4(x[4 * h], x[4 * h + 1], x[4 * h + 2], x[4 * h + 3]));
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int j = jj + k;
-            if (j < n && i <= j) __stcs(orow + j, (i == j) ? 0.0f : x[4 * h + k]);
-          }
-        }
+      for (int k = 0; k < 8; ++k) {
+        const int j = j0 + k;
+        if (j < n && i <= j) __stcs(rp + k, (i == j) ? 0.0f : x[k]);
       }
     }
-    // The next group's counts into registers 0 .. 7.
-#pragma unroll
-    for (int k = 0; k < 32 - kTcfGroup; ++k) pq[k] = pq[k + kTcfGroup];
-#pragma unroll
-    for (int k = 0; k < (32 - kTcfGroup) / 2; ++k) pv[k] = pv[k + kTcfGroup / 2];
   }
 }
 
-// Kimura-2P rows (the variant of the DNA workloads): the 32 distances of row i,
-// columns jb .. jb + 31, in groups of four computed without branches
-// (k2p_decide16), the rare undecided pairs out of line; stores as streaming
-// stores (.cs), so that the output does not push the logarithm table out of
-// L1.  interior: the tile lies above the diagonal and inside the matrix (every
-// pair valid, no masks).
-constexpr int kK2pGroups = 4;  // groups of four pairs computed per loop iteration
+// The valid count of column k of a pair of packed 16-bit counts, plus 2^23: the
+// 16 bits under that exponent.
+__device__ __forceinline__ float valid23_of(uint32_t pv, int k) {
+  return __uint_as_float(__byte_perm(pv, 0x4B000000u, (k & 1) ? 0x7432 : 0x7410));
+}
+__device__ __forceinline__ float valid_of(uint32_t pv, int k) {
+  return __fsub_rn(valid23_of(pv, k), 8388608.0f);
+}
 
-__device__ __forceinline__ void fused_rows_k2p(const AlnDesc &d, int i, int jb, bool interior,
-                                               uint32_t (&pq)[32], uint32_t (&pv)[16],
-                                               float &tmax, bool &sat, const double2 *tab) {
-  const int n = d.n;
-  float *const out = d.out;
-  const size_t ld = d.ld;
-  const bool vec = ((ld & 3) == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
-  float *const orow = out + (size_t)i * ld;  // dereferenced only for i < n
-  float *mp = out + (size_t)jb * ld + i;     // out[jb + c][i], one row further per column
-  constexpr int U = kK2pGroups;
-#pragma unroll 1
-  for (int it = 0; it < 8 / U; ++it) {
+// Sixteen columns of row i, from jb: pv the valid counts (two a word), ar and at
+// the other accumulators' words.  Eight at a time: a group of the warp's rows and
+// eight columns lies above the diagonal and inside the matrix (no masks), or
+// holds nothing of the triangle (skipped), or straddles an edge.
+template <int M, bool kProt>
+__device__ __forceinline__ void fused_cols(const AlnDesc &d, float *out, size_t ld, int n, int i,
+                                           int jb, RowStore how, const uint32_t (&pv)[16], const uint32_t (&ar)[16],
+                                           const uint32_t (&at)[16], float &tmax, float &tmin,
+                                           double inv_b, const RoundCheck &rc,
+                                           const TcfTables &tab) {
+  const int ilo = i - (int)(threadIdx.x & 31);  // the warp's first row
 #pragma unroll
-  for (int g = 0; g < U; ++g) {
+  for (int g = 0; g < 2; ++g) {
+    const int j0 = jb + 8 * g;
+    if (j0 + 7 < ilo || j0 >= n || ilo >= n) continue;
+    const bool interior = ilo + 31 < j0 && j0 + 7 < n && (ld >> 32) == 0;
+    float x[8];
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      const int c = 8 * g + k;
+      const uint32_t v = pv[c >> 1];
+      if constexpr (M == kFusedGeneric) {
+        x[k] = generic_pair(d, valid_of(v, 0), __uint_as_float(ar[c]), __uint_as_float(at[c]));
+        x[k + 1] = generic_pair(d, valid_of(v, 1), __uint_as_float(ar[c + 1]),
+                                __uint_as_float(at[c + 1]));
+      } else {
+        bool s0 = false, s1 = false;
+        fused_pair2<M, kProt>(pack2(valid23_of(v, 0), valid23_of(v, 1)),
+                              pack2(__uint_as_float(ar[c]), __uint_as_float(ar[c + 1])),
+                              pack2(__uint_as_float(at[c]), __uint_as_float(at[c + 1])), inv_b, rc,
+                              tab, x[k], x[k + 1], s0, s1);
+        any |= s0 | s1;
+      }
+    }
+    if constexpr (M != kFusedGeneric) {
+      if (any) {
+#pragma unroll 1
+        for (int k = 0; k < 8; ++k) {
+          // (a second pass finds the undecided ones again: no flags are kept)
+          bool slow = false, other = false;
+          float fv = 0.0f, fr = 0.0f, ft = 0.0f, x0, x1;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            if (u != k) continue;
+            fv = valid_of(pv[(8 * g + u) >> 1], u);
+            fr = __uint_as_float(ar[8 * g + u]);
+            ft = __uint_as_float(at[8 * g + u]);
+          }
+          const float v23 = __fadd_rn(fv, 8388608.0f);
+          fused_pair2<M, kProt>(pack2(v23, v23), pack2(fr, fr), pack2(ft, ft), inv_b, rc, tab, x0,
+                                x1, slow, other);
+          if (!slow) continue;
+          const float v = fused_undecided<M, kProt>(fv, fr, ft);
+#pragma unroll
+          for (int u = 0; u < 8; ++u) x[u] = u == k ? v : x[u];
+        }
+      }
+    }
+    if (!interior) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[k] = (i < j0 + k && j0 + k < n) ? x[k] : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      tmax = max3(tmax, x[k], x[k + 1]);
+      tmin = min3(tmin, x[k], x[k + 1]);
+    }
+    store_group(out, ld, n, i, j0, interior, how, x, tab.stage);
+  }
+}
+
+// Full-rows form (a band of full-square tiles, AlnDesc::full): sixteen columns of
+// row i from jb, every j != i (0 on the diagonal), into row i - row0 of the band
+// buffer; no mirror.
+__device__ __forceinline__ void fused_cols_full(const AlnDesc &d, int i, int jb,
+                                                const uint32_t (&pv)[16],
+                                                const uint32_t (&ar)[16], const uint32_t (&at)[16],
+                                                float &tmax, float &tmin) {
+  const int n = d.n;
+  const size_t ld = d.ld;
+  float *const orow = d.out + (size_t)(i - d.row0) * ld;  // dereferenced only for i < n
+  const bool vec = ((ld & 3) == 0) && ((reinterpret_cast<uintptr_t>(d.out) & 15) == 0);
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    const int j0 = jb + 4 * g;
     float x[4];
-    uint32_t undecided = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int c = 4 * g + k;
-      bool slow;
-      x[k] = k2p_decide16(pq[c] & 0xFFFFu, pq[c] >> 16, (pv[c >> 1] >> (16 * (c & 1))) & 0xFFFFu,
-                          slow, tab);
-      undecided |= (uint32_t)slow << k;
+      const int j = j0 + k, c = 4 * g + k;
+      x[k] = 0.0f;
+      if (i < n && j != i && j < n)
+        x[k] = generic_pair(d, valid_of(pv[c >> 1], c), __uint_as_float(ar[c]),
+                            __uint_as_float(at[c]));
+      tmax = fmaxf(tmax, x[k]);
+      tmin = fminf(tmin, x[k]);
     }
-    if (undecided) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int c = 4 * g + k;
-        if ((undecided >> k) & 1u)
-          x[k] = k2p_undecided(pq[c] & 0xFFFFu, pq[c] >> 16,
-                               (pv[c >> 1] >> (16 * (c & 1))) & 0xFFFFu);
-      }
-    }
-    const int j0 = jb + 4 * (U * it + g);
-    if (interior) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        tmax = fmaxf(tmax, x[k]);
-        sat |= (x[k] == -1.0f);
-        __stcs(mp, x[k]);  // mirror: consecutive i across lanes
-        mp += ld;
-      }
-      if (vec) {
-        __stcs(reinterpret_cast<float4 *>(orow + j0), make_float4(x[0], x[1], x[2], x[3]));
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) __stcs(orow + j0 + k, x[k]);
-      }
+    if (i >= n) continue;
+    if (vec && j0 + 3 < n) {
+      __stcs(reinterpret_cast<float4 *>(orow + j0), make_float4(x[0], x[1], x[2], x[3]));
     } else {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int j = j0 + k;
-        const bool in = i < j && j < n;
-        x[k] = in ? x[k] : 0.0f;
-        tmax = fmaxf(tmax, x[k]);
-        sat |= (x[k] == -1.0f);
-        if (in) __stcs(mp, x[k]);
-        mp += ld;
-      }
-      if (i < n) {
-        if (vec && i < j0 && j0 + 3 < n) {
-          __stcs(reinterpret_cast<float4 *>(orow + j0), make_float4(x[0], x[1], x[2], x[3]));
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int j = j0 + k;
-            if (j < n && i <= j) __stcs(orow + j, (i == j) ? 0.0f : x[k]);
-          }
-        }
-      }
+      for (int k = 0; k < 4; ++k)
+        if (j0 + k < n) __stcs(orow + j0 + k, x[k]);
     }
-  }
-  // The next iteration's counts into registers 0 .. 4U - 1.
-  if constexpr (U < 8) {
-#pragma unroll
-    for (int k = 0; k < 32 - 4 * U; ++k) pq[k] = pq[k + 4 * U];
-#pragma unroll
-    for (int k = 0; k < 16 - 2 * U; ++k) pv[k] = pv[k + 2 * U];
-  }
   }
 }
 
-// Full-rows form (a band of full-square tiles, AlnDesc::full): the 32
-// distances of row i, columns jb .. jb + 31, every j != i (0 on the diagonal),
-// into row i - row0 of the band buffer; no mirror.
-template <int M>
-__device__ __forceinline__ void fused_rows_full(const AlnDesc &d, int i, int jb, uint32_t (&pq)[32],
-                                                uint32_t (&pv)[16], float &tmax, bool &sat) {
-  const int n = d.n;
-  if (i >= n) return;
-  const size_t ld = d.ld;
-  float *const orow = d.out + (size_t)(i - d.row0) * ld;
-  const bool vec = ((ld & 3) == 0) && ((reinterpret_cast<uintptr_t>(d.out) & 15) == 0);
-#pragma unroll 1
-  for (int g = 0; g < 32 / kTcfGroup; ++g) {
-    const int j0 = jb + kTcfGroup * g;
-    float x[kTcfGroup];
-#pragma unroll
-    for (int k = 0; k < kTcfGroup; ++k) {
-      const int j = j0 + k;
-      x[k] = 0.0f;
-      if (j != i && j < n) {
-        const uint32_t vv = (pv[k >> 1] >> (16 * (k & 1))) & 0xFFFFu;
-        x[k] = fused_pair<M>(d, pq[k] & 0xFFFFu, pq[k] >> 16, vv);
-        tmax = fmaxf(tmax, x[k]);
-        sat |= (x[k] == -1.0f);
-      }
-    }
-#pragma unroll
-    for (int h = 0; h < kTcfGroup / 4; ++h) {
-      const int jj = j0 + 4 * h;
-      if (vec && jj + 3 < n) {
-        __stcs(reinterpret_cast<float4 *>(orow + jj),
-               make_float4(x[4 * h], x[4 * h + 1], x[4 * h + 2], x[4 * h + 3]));
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (jj + k < n) __stcs(orow + jj + k, x[4 * h + k]);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 32 - kTcfGroup; ++k) pq[k] = pq[k + kTcfGroup];
-#pragma unroll
-    for (int k = 0; k < (32 - kTcfGroup) / 2; ++k) pv[k] = pv[k + kTcfGroup / 2];
-  }
+// An epilogue warp has read part k of the accumulators (the leader's MMA warp
+// waits for both CTAs' warps).
+template <bool kPair>
+__device__ __forceinline__ void arrive_read(const TcShared &sh, int k) {
+  if (kPair) mbar_arrive_cluster(cluster_addr(&sh.tmem_empty[k], 0));
+  else mbar_arrive(&sh.tmem_empty[k]);
 }
 
-// One tile of the epilogue (every epilogue warp; warp w reads tensor-memory
-// lane quarter w % 4 and columns 32 (w / 4) .. + 31): waits for the
-// accumulators of the CTA's item number titer, reads them, hands tensor memory
-// back, then the transform, the stores, the tile's maximum and saturation
-// flag.  False when a wait ran out (the caller sets the abort flag).
-template <int V>
-__device__ __forceinline__ bool fused_tile(const TcShared &sh, uint32_t tmem, const AlnDesc &d,
-                                           int tile, uint32_t titer, int stall, uint64_t limit,
-                                           const double2 *tab, int *sat_any = nullptr) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q = warp & 3;              // tensor-memory lane quarter
-  const int cofs = 32 * (warp >> 2);   // first tile column of this warp
-  const int row = 32 * q + lane;       // tile row of this lane
-  int ti, tj;
-  item_tile(d, tile, ti, tj);
-  if ((stall && titer == 0 && !tc_wait(sh.never_bar, 0, sh.abort_flag, limit)) ||
-      !tc_wait(sh.acc_full, titer & 1, sh.abort_flag, limit))
-    return false;
-  tc_fence_after();
-  // protein counts (V - M) or DNA (ts, tv): known at compile time for the
-  // single-model variants (K2P is DNA, protein Kimura is protein)
-  const bool prot = V == kFusedK2p ? false
-                                   : (V == kFusedProtein ? true : d.kind == KIND_PROT_TC);
-  // Accumulators -> integer counts (DNA: transitions, transversions, valid;
-  // protein: mismatches = V - M, 0, valid), 16 columns at a time, 16 bits
-  // each (the fused form takes L < 65536): pq[k] = ts | tv << 16, and the
-  // valid counts two to a register.
-  uint32_t pq[32], pv[16];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    uint32_t av[16], ar[16], at[16];  // accumulators V, R, T
-    const uint32_t base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(cofs + 16 * h);
-    tmem_ld16(base, av);
-    tmem_ld16(base + kTile, ar);
-    tmem_ld16(base + 2 * kTile, at);
-    tmem_ld_wait();
-    // The sums are exact integers in f32 (below 2^24 in magnitude), and so
-    // are P = (V + R - T) / 4 and Q = (V - R) / 2 (DNA) or P = V - M
-    // (protein); x + 2^23 holds x in its low mantissa bits (0 <= x < 2^23),
-    // from which the 16-bit fields are taken without a conversion.
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const float fv = __uint_as_float(av[k]), fr = __uint_as_float(ar[k]);
-      const float ft = __uint_as_float(at[k]);
-      // DNA: 4P = V + R - T and 2Q = V - R are exact integers, so the scale and
-      // the bias fuse into one multiply-add with the same (exact) result.
-      const uint32_t bp = __float_as_uint(
-          prot ? __fadd_rn(__fsub_rn(fv, fr), 8388608.0f)
-               : __fmaf_rn(__fsub_rn(__fadd_rn(fv, fr), ft), 0.25f, 8388608.0f));
-      const uint32_t bq = __float_as_uint(
-          prot ? 8388608.0f : __fmaf_rn(__fsub_rn(fv, fr), 0.5f, 8388608.0f));
-      const uint32_t bv = __float_as_uint(__fadd_rn(fv, 8388608.0f));
-      pq[16 * h + k] = __byte_perm(bp, bq, 0x5410);  // P | Q << 16
-      if (k & 1) pv[8 * h + (k >> 1)] = __byte_perm(pv[8 * h + (k >> 1)], bv, 0x5410);
-      else pv[8 * h + (k >> 1)] = bv;  // high half replaced by the odd column
-    }
-  }
-  // Tensor memory back to the MMA warp: the next tile's MMAs start now.
-  tc_fence_before();
-  __syncwarp();
-  if (lane == 0) mbar_arrive(sh.tmem_empty);
-
-  const int i = ti * kTile + row;
-  const int jb = tj * kTile + cofs;
-  float tmax = 0.0f;
-  bool sat = false;
-  if constexpr (V == kFusedFull) {
-    // a band of full rows (out-of-core delivery), every model
-    fused_rows_full<kFusedGeneric>(d, i, jb, pq, pv, tmax, sat);
-  } else if constexpr (V == kFusedK2p) {
-    fused_rows_k2p(d, i, jb, ti < tj && (tj + 1) * kTile <= d.n, pq, pv, tmax, sat, tab);
-  } else if constexpr (V != kFusedAny) {
-    fused_rows<V>(d, i, jb, pq, pv, tmax, sat, tab);
-  } else if (d.compat) {
-    fused_rows<kFusedGeneric>(d, i, jb, pq, pv, tmax, sat, tab);
-  } else if (d.model == RNJ_JC) {
-    fused_rows<kFusedJc>(d, i, jb, pq, pv, tmax, sat, tab);
-  } else if (d.type == RNJ_PROTEIN) {
-    fused_rows<kFusedProtein>(d, i, jb, pq, pv, tmax, sat, tab);
-  } else {
-    fused_rows_k2p(d, i, jb, ti < tj && (tj + 1) * kTile <= d.n, pq, pv, tmax, sat, tab);
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-    tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, off));
-  const bool any_sat = __any_sync(0xffffffffu, sat);
-  if (lane == 0) {
-    if (tmax > 0.0f) atomicMax(d.max_bits, __float_as_int(tmax));
-    if (any_sat) {
-      d.tile_flags[tile] = 1;
-      if (sat_any) atomicOr(sat_any, 1);
-    }
+// The part of a CTA of a pair that has no tile of the item: its accumulators are
+// handed back unread.
+__device__ __forceinline__ bool skip_tile(const TcShared &sh, uint32_t titer, int stall,
+                                          uint64_t limit) {
+  if (stall && titer == 0 && !tc_wait(sh.never_bar, 0, sh.abort_flag, limit)) return false;
+  for (int k = 0; k < 2; ++k) {
+    if (!tc_wait(&sh.acc_full[k], titer & 1, sh.abort_flag, limit)) return false;
+    if ((threadIdx.x & 31) == 0) arrive_read<true>(sh, k);
+    __syncwarp();
   }
   return true;
 }
 
+// One tile of the epilogue (every epilogue warp; warp w reads tensor-memory
+// lane quarter w % 4 and columns 32 (w / 4) .. + 31): waits for V of the CTA's
+// item number titer and hands it back, then for the other accumulators, which
+// go back once their second half is in registers; the transform, the stores,
+// the tile's maximum (through the alignment's max slot when it exceeds `seen`,
+// the largest this warp has sent there) and saturation flag.  False when a wait
+// ran out (the caller sets the abort flag).
+template <int M, bool kProt, bool kPair>
+__device__ __forceinline__ bool fused_tile_as(const TcShared &sh, uint32_t tmem, const AlnDesc &d,
+                                           const TileAt &t, uint32_t titer, int stall,
+                                           uint64_t limit, const TcfTables &tab, float &seen,
+                                           int *sat_any = nullptr) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q = warp & 3;              // tensor-memory lane quarter
+  const int cofs = 32 * (warp >> 2);   // first tile column of this warp
+  const int i = t.ti * kTile + 32 * q + lane;  // this lane's row
+  const int jb = t.tj * kTile + cofs;
+  const uint32_t base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)cofs;
+  // The descriptor's fields, read once (every store below could have changed
+  // them, for all the compiler knows).
+  float *const out = d.out;
+  const size_t ld = d.ld;
+  const int n = d.n;
+  const RoundCheck rc(margin<M>(d.L));
+  const uintptr_t oa = reinterpret_cast<uintptr_t>(out);
+  const RowStore how = ((ld & 7) == 0 && (oa & 31) == 0)
+                           ? kRowVec8
+                           : (((ld & 3) == 0 && (oa & 15) == 0) ? kRowVec4 : kRowStaged);
+  const double inv_b = M == kFusedJc ? 1.0 / (kProt ? 0.95 : 0.75) : 0.0;
+  if ((stall && titer == 0 && !tc_wait(sh.never_bar, 0, sh.abort_flag, limit)) ||
+      !tc_wait(&sh.acc_full[0], titer & 1, sh.abort_flag, limit))
+    return false;
+  tc_fence_after();
+  // V: exact integers below 2^16; v + 2^23 holds v in its low mantissa bits, two
+  // of which go into a word.
+  uint32_t pv[16];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t av[16];
+    tmem_ld16(base + 16 * h, av);
+    tmem_ld_wait();
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      pv[8 * h + k] = __byte_perm(
+          __float_as_uint(__fadd_rn(__uint_as_float(av[2 * k]), 8388608.0f)),
+          __float_as_uint(__fadd_rn(__uint_as_float(av[2 * k + 1]), 8388608.0f)), 0x5410);
+  }
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) arrive_read<kPair>(sh, 0);  // the next tile's V may start
+  if (!tc_wait(&sh.acc_full[1], titer & 1, sh.abort_flag, limit)) return false;
+  tc_fence_after();
+
+  float tmax = 0.0f, tmin = 0.0f;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    uint32_t ar[16], at[16];
+    tmem_ld16(base + kTile + 16 * h, ar);
+    tmem_ld16(base + 2 * kTile + 16 * h, at);
+    tmem_ld_wait();
+    if (h == 1) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) arrive_read<kPair>(sh, 1);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) pv[k] = pv[k + 8];
+    }
+    const int jh = jb + 16 * h;
+    if constexpr (M == kFusedFull)
+      fused_cols_full(d, i, jh, pv, ar, at, tmax, tmin);
+    else
+      fused_cols<M, kProt>(d, out, ld, n, i, jh, how, pv, ar, at, tmax, tmin, inv_b, rc,
+                           tab);
+  }
+  // (non-negative floats order as their bits)
+  tmax = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(tmax)));
+  const bool any_sat = __any_sync(0xffffffffu, tmin < 0.0f);
+  if (lane == 0) {
+    if (tmax > seen) atomicMax(d.max_bits, __float_as_int(tmax));
+    if (any_sat) {
+      d.tile_flags[t.tile] = 1;
+      if (sat_any) atomicOr(sat_any, 1);
+    }
+  }
+  seen = fmaxf(seen, tmax);
+  return true;
+}
+
+// The tile by its variant: each model's code on its own, so that none keeps
+// another's parameters in registers.
+template <int V, bool kPair>
+__device__ __forceinline__ bool fused_tile(const TcShared &sh, uint32_t tmem, const AlnDesc &d,
+                                           const TileAt &t, uint32_t titer, int stall,
+                                           uint64_t limit, const TcfTables &tab, float &seen,
+                                           int *sat_any = nullptr) {
+#define RNJ_TILE(M, P) \
+  fused_tile_as<M, P, kPair>(sh, tmem, d, t, titer, stall, limit, tab, seen, sat_any)
+  if constexpr (V == kFusedFull) return RNJ_TILE(kFusedFull, false);
+  else if constexpr (V == kFusedK2p) return RNJ_TILE(kFusedK2p, false);
+  else if constexpr (V == kFusedProtein) return RNJ_TILE(kFusedProtein, true);
+  else if constexpr (V == kFusedGeneric) return RNJ_TILE(kFusedGeneric, false);
+  else {
+    const bool prot = d.kind == KIND_PROT_TC;
+    if (V == kFusedAny && d.compat) return RNJ_TILE(kFusedGeneric, false);
+    if (V == kFusedJc || d.model == RNJ_JC)
+      return prot ? RNJ_TILE(kFusedJc, true) : RNJ_TILE(kFusedJc, false);
+    return prot ? RNJ_TILE(kFusedProtein, true) : RNJ_TILE(kFusedK2p, false);
+  }
+#undef RNJ_TILE
+}
+
 // V: the transform variant of every item (kFused*), or kFusedAny to choose per
-// item (a work list of alignments with different models).
+// item (a work list of alignments with different models).  Items [first, last),
+// one per pair of CTAs at a time.
 template <int V>
-__global__ void __launch_bounds__(kTcfThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcfThreads, 1)
     tc_fused_kernel(const AlnDesc *__restrict__ descs, const WorkItem *__restrict__ items,
-                    const int *__restrict__ nitems_ptr, int nitems_direct, int item0, int count,
-                    int nst) {
+                    int first, int nitems, int nst) {
   extern __shared__ uint8_t smem_raw[];
-  // A batch's first descriptor may ask for a shallower ring than the launch's
-  // shared memory holds (its graph is captured once; batches launch kFusedAny).
-  if constexpr (V == kFusedAny)
-    if (descs[0].stages > 0) nst = max(kTcMinStages, min(nst, descs[0].stages));
-  const TcShared sh = tc_shared(smem_raw, nst, kTcfTableBytes);
-  double2 *const tab = reinterpret_cast<double2 *>(tc_extra(sh));
+  const TcShared sh = tc_shared(smem_raw, nst, kTcfExtra);
   const uint64_t limit = wait_limit_ns((uint32_t)descs[0].wait_us);
   const int stall = descs[0].stall;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // items [item0, min(nitems, item0 + count))
-  const int nitems = (int)min((long long)(nitems_ptr ? *nitems_ptr : nitems_direct),
-                              (long long)item0 + count);
-  const int it0 = item0 + (int)blockIdx.x;
-  if (it0 >= nitems) return;  // no item for this CTA (before any setup)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank();
+  const int it0 = first + (int)(blockIdx.x >> 1), step = (int)(gridDim.x >> 1);
+  if (it0 >= nitems) return;  // no item for this pair (both CTAs, before any setup)
 
-  for (int e = tid; e < 128; e += kTcfThreads)
-    tab[e] = make_double2(-0.25 * c_log_tab[e][0], -0.25 * c_log_tab[e][1]);
-  // tmem_empty: one arrival per epilogue warp; the scale factors by warps 0 .. 7
-  const uint32_t tmem = tc_setup(sh, kTcfEpiWarps, 0, kTcfMmaWarp);
-  uint32_t issued = 0;
+  const TcfTables tab = tcf_tables(sh);
+  const uint32_t tmem = pair_setup(sh, kTcfEpiWarps, kTcfMmaWarp);
 
   if (warp >= kTcfProducerWarp) {
     // The register split is made inside each role's branch, so that the
     // compiler allocates each role's code within its own limit.
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kTcfRegsLow) : "memory");
     if (warp == kTcfProducerWarp) {
-      if (lane == 0) issued = tc_produce(sh, descs, items, it0, nitems, gridDim.x, limit);
-    } else if (warp == kTcfMmaWarp) {
-      tc_issue(sh, tmem, descs, items, it0, nitems, gridDim.x, limit);
+      if (lane == 0) pair_produce(sh, rank, descs, items, it0, nitems, step, limit);
+    } else if (warp == kTcfMmaWarp && rank == 0) {
+      pair_issue(sh, tmem, descs, items, it0, nitems, step, limit);
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kTcfRegsHigh) : "memory");
     // ----------------------------------------------------------- epilogue
     uint32_t titer = 0;
-    for (int it = it0; it < nitems; it += gridDim.x, ++titer) {
-      const WorkItem w = item_at(descs, items, it);
-      if (!fused_tile<V>(sh, tmem, descs[w.aln], w.tile, titer, stall, limit, tab)) {
-        *sh.abort_flag = 1;
+    PairWalk walk(descs, items, rank);
+    float seen = 0.0f;
+    int last = 0;
+    for (int it = it0; it < nitems; it += step, ++titer) {
+      const TileAt t = walk.at(it);
+      if (t.aln != last) {
+        last = t.aln;
+        seen = 0.0f;
+      }
+      const bool ok = t.tile < 0
+                          ? skip_tile(sh, titer, stall, limit)
+                          : fused_tile<V, true>(sh, tmem, descs[t.aln], t, titer, stall, limit,
+                                                tab, seen);
+      if (!ok) {
+        pair_abort(sh);
         break;
       }
     }
   }
 
-  tc_teardown(sh, tmem, issued, descs[0].err, kTcfMmaWarp);
+  pair_teardown(sh, rank, tmem, descs[0], descs[0].err, kTcfMmaWarp);
 }
 
 // ------------------------------------------------------------ live form
@@ -465,7 +650,8 @@ struct LiveRing {
   int last;      // the item just finished completes its request's tiles
   int sat;       // ... and one of them holds a saturated pair
 };
-constexpr size_t kLiveExtra = kTcfTableBytes + 128;
+constexpr size_t kLiveExtra = kTcfExtra + 128;
+static_assert(tc_smem_bytes(kTcfStages, kLiveExtra) <= 232448, "fits the shared memory of one CTA");
 static_assert(sizeof(LiveRing) <= 128, "the live ring fits its shared-memory slot");
 constexpr int kLiveFix = 0x40000000;  // WorkItem::aln bit of a fix-up item in the ring
 
@@ -586,13 +772,11 @@ __global__ void __launch_bounds__(kTcfThreads, 1)
     tc_live_kernel(const AlnDesc *__restrict__ descs, const LiveList live, int nst) {
   extern __shared__ uint8_t smem_raw[];
   const TcShared sh = tc_shared(smem_raw, nst, kLiveExtra);
-  double2 *const tab = reinterpret_cast<double2 *>(tc_extra(sh));
-  LiveRing *const lr = reinterpret_cast<LiveRing *>(tc_extra(sh) + kTcfTableBytes);
+  LiveRing *const lr = reinterpret_cast<LiveRing *>(tc_extra(sh) + kTcfExtra);
   const uint64_t limit = wait_limit_ns((uint32_t)descs[0].wait_us);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  for (int e = tid; e < 128; e += kTcfThreads)
-    tab[e] = make_double2(-0.25 * c_log_tab[e][0], -0.25 * c_log_tab[e][1]);
+  const TcfTables tab = tcf_tables(sh);
   if (tid == 0) {
     for (int k = 0; k < 2; ++k) {
       mbar_init(&lr->full[k], 1);
@@ -637,7 +821,9 @@ __global__ void __launch_bounds__(kTcfThreads, 1)
         }
         if (w.aln < 0) break;
         if (w.aln & kLiveFix) continue;  // the epilogue warps' work only
-        if (!tc_produce_item(sh, descs[w.aln], w.tile, gkb, issued, ps, pph, limit)) break;
+        int ti, tj;
+        item_tile(descs[w.aln], w.tile, ti, tj);
+        if (!tc_produce_item(sh, descs[w.aln], ti, tj, gkb, issued, ps, pph, limit)) break;
       }
     } else if (warp == kTcfMmaWarp) {
       // ------------------------------------------------------- MMA issuer
@@ -719,7 +905,11 @@ __global__ void __launch_bounds__(kTcfThreads, 1)
         continue;
       }
       // ----------------------------------------------- a tile to compute
-      if (!fused_tile<kFusedAny>(sh, tmem, d, tile, titer, 0, limit, tab, &live.sat[aln])) {
+      TileAt t{aln, tile, 0, 0};
+      item_tile(d, tile, t.ti, t.tj);
+      float seen = 0.0f;
+      if (!fused_tile<kFusedAny, false>(sh, tmem, d, t, titer, 0, limit, tab, seen,
+                                       &live.sat[aln])) {
         *sh.abort_flag = 1;
         break;
       }
@@ -819,17 +1009,49 @@ cudaError_t launch_live_publish(const LiveList &live, int aln, int nt, int band,
   return cudaGetLastError();
 }
 
+// Pairs of CTAs that run at one time (one CTA per SM; a cluster needs two SMs of
+// one GPC), per device.
+static int max_pairs(int device, cudaError_t *err) {
+  static std::atomic<int> known[64];
+  const bool keep = device >= 0 && device < 64;
+  if (keep && known[device].load(std::memory_order_relaxed) > 0)
+    return known[device].load(std::memory_order_relaxed);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 2;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(2);
+  cfg.blockDim = dim3(kTcfThreads);
+  cfg.dynamicSmemBytes = kTcfSmemBytes;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  *err = cudaOccupancyMaxActiveClusters(&n, tc_fused_kernel<kFusedK2p>, &cfg);
+  if (*err != cudaSuccess) return 0;
+  n = std::max(1, n);
+  if (keep) known[device].store(n, std::memory_order_relaxed);
+  return n;
+}
+
 template <int V>
 static cudaError_t launch_variant(const AlnDesc *d_descs, const WorkItem *d_items,
-                                  const int *d_nitems, int nitems, int item0, int count, int grid,
-                                  int stages, cudaStream_t s) {
-  const int nst = tc_ring_depth(stages, kTcfStages, kTcfStages);
-  const size_t smem = tc_smem_bytes(nst, kTcfTableBytes);
-  cudaError_t e = cudaFuncSetAttribute(tc_fused_kernel<V>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                  int first, int count, int stages, cudaStream_t s) {
+  const int nst = pair_stages(stages);
+  const size_t smem = tc_smem_bytes(nst, kTcfExtra, kPairStageBytes);
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(tc_fused_kernel<kFusedK2p>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcfSmemBytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(tc_fused_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kTcfSmemBytes);
   if (e != cudaSuccess) return e;
-  tc_fused_kernel<V><<<(unsigned)grid, kTcfThreads, smem, s>>>(d_descs, d_items, d_nitems, nitems,
-                                                              item0, count, nst);
+  const int pairs = std::min(count, max_pairs(device, &e));
+  if (e != cudaSuccess) return e;
+  tc_fused_kernel<V><<<(unsigned)(2 * pairs), kTcfThreads, smem, s>>>(
+      d_descs, d_items, first, first + count, nst);
   return cudaGetLastError();
 }
 
@@ -842,18 +1064,53 @@ int fused_variant_for(int model, int type, int compat, int full) {
 
 int fused_ring_depth(int stages) { return tc_ring_depth(stages, kTcfStages, kTcfStages); }
 
-cudaError_t launch_tc_fused(const AlnDesc *d_descs, const WorkItem *d_items, const int *d_nitems,
-                            int nitems, int item0, int count, int grid, int variant,
-                            cudaStream_t s, int stages) {
-  if (grid <= 0) return cudaSuccess;
-  using Launch = cudaError_t (*)(const AlnDesc *, const WorkItem *, const int *, int, int, int,
-                                 int, int, cudaStream_t);
+cudaError_t launch_tc_fused(const AlnDesc *d_descs, const WorkItem *d_items, int first, int count,
+                            int variant, cudaStream_t s, int stages) {
+  if (count <= 0) return cudaSuccess;
+  using Launch = cudaError_t (*)(const AlnDesc *, const WorkItem *, int, int, int, cudaStream_t);
   // indexed by FusedVariant
-  static const Launch kLaunch[] = {launch_variant<kFusedK2p>,     launch_variant<kFusedJc>,
+  static const Launch kLaunch[] = {launch_variant<kFusedK2p>, launch_variant<kFusedJc>,
                                    launch_variant<kFusedProtein>, launch_variant<kFusedGeneric>,
-                                   launch_variant<kFusedFull>,    launch_variant<kFusedAny>};
+                                   launch_variant<kFusedFull>, launch_variant<kFusedAny>};
   if (variant < FUSED_K2P || variant > FUSED_ANY) return cudaErrorInvalidValue;
-  return kLaunch[variant](d_descs, d_items, d_nitems, nitems, item0, count, grid, stages, s);
+  return kLaunch[variant](d_descs, d_items, first, count, stages, s);
+}
+
+long long pair_items(int nt) {
+  const long long p = (nt + 1) / 2;
+  return p * nt - p * (p - 1);
+}
+
+// Work items of tile rows [r0, r1) of a triangle, columns tj >= r0 (those of a
+// band of the streamed call), column by column: a row pair for every two rows
+// of the band, a single for an odd one.
+void pair_items_of_band(int aln, int nt, int r0, int r1, std::vector<WorkItem> &out) {
+  for (int tj = r0; tj < nt; ++tj)
+    for (int ti = r0; ti < r1 && ti <= tj; ti += 2)
+      out.push_back(WorkItem{aln, tri_index(ti, tj, nt) | (ti + 1 < r1 ? 0 : kPairSingle)});
+}
+
+// The same for tiles [t0, t1) of the row-major triangle order (a shard).
+void pair_items_of_range(int aln, int nt, long long t0, long long t1, std::vector<WorkItem> &out) {
+  auto start = [&](long long r) { return r * nt - r * (r - 1) / 2; };
+  auto cols = [&](int r, int &c0, int &c1) {  // the range's columns of tile row r
+    const long long a = std::max(t0, start(r)), b = std::min(t1, start(r + 1));
+    c0 = r + (int)(a - start(r));
+    c1 = a < b ? r + (int)(b - start(r)) : c0;
+  };
+  for (int ti = 0; ti < nt; ti += 2) {
+    if (start(std::min(ti + 2, nt)) <= t0) continue;
+    if (start(ti) >= t1) break;
+    int a0, a1, b0 = 0, b1 = 0;
+    cols(ti, a0, a1);
+    if (ti + 1 < nt) cols(ti + 1, b0, b1);
+    for (int tj = ti; tj < nt; ++tj) {
+      const bool a = tj >= a0 && tj < a1, b = tj >= b0 && tj < b1;
+      // (tj = ti: the second row's tile lies below the diagonal)
+      if (a) out.push_back(WorkItem{aln, tri_index(ti, tj, nt) | (b || tj == ti ? 0 : kPairSingle)});
+      else if (b) out.push_back(WorkItem{aln, tri_index(ti + 1, tj, nt) | kPairSingle});
+    }
+  }
 }
 
 }  // namespace rnj
