@@ -190,8 +190,9 @@ int rnj_counts_into(rnj_ctx *ctx, rnj_aln *aln, unsigned int *d_counts);
  * in double (KimuraDistance.cpp:366-395): saturated pairs (-1) become twice
  * the maximum of the doubles, the lower triangle mirrors the upper (full rows
  * with RNJ_FULL_ROWS), the diagonal is 0.  max_out (may be NULL) receives that
- * maximum.  Synchronous.  Scratch: the n x n x 3 counts (12 n^2 bytes), freed
- * before the call returns.  No counterpart in the reference, whose matrix is
+ * maximum.  Synchronous.  Scratch: 128 KB per 128 x 128 tile of the triangle, at
+ * most 512 MiB, kept by the context (tensor-core layouts), or the n x n x 3 counts
+ * (12 n^2 bytes), freed before the call returns (bit planes).  No counterpart in the reference, whose matrix is
  * float; (float) of each value is the reference's entry. */
 int rnj_distance_f64(rnj_ctx *ctx, rnj_aln *aln, int model, double *d_out, size_t ld,
                      double *max_out);

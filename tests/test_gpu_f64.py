@@ -114,3 +114,28 @@ def test_double_matrix_rejects_bad_arguments(ctx):
     with pytest.raises(RnjError):
         ctx.distance_f64(aln, "kim", out=small)
     aln.close()
+
+
+@pytest.mark.parametrize("n,L", [(31, 40), (129, 300), (255, 257), (641, 100), (12000, 64)])
+@pytest.mark.parametrize("typ,model", [(0, "kim"), (0, "jc"), (1, "kim")])
+def test_tiles_and_passes(ctx, n, L, typ, model):
+    from rapidnj_b200 import synth
+    # Edge tiles, a strided output, and more tiles than one pass of packed counts
+    # holds (12,000 rows): the doubles' floats are the float matrix (one ulp where
+    # a logarithm's double rounding decides), symmetric, nothing outside written.
+    if n > 1000 and model == "jc":
+        pytest.skip("one model at the large size")
+    s = (synth.tree_dna if typ == 0 else synth.tree_protein)(min(n, 700), L, seed=n)
+    s = np.ascontiguousarray(s[np.arange(n) % s.shape[0]])
+    aln = ctx.alignment(s, typ)
+    flt = torch.empty((n, n), dtype=torch.float32, device="cuda")
+    ctx.distance_into(aln, model, flt)
+    buf = torch.full((n, n + 3), -7.0, dtype=torch.float64, device="cuda")
+    out, mx = ctx.distance_f64(aln, model, buf)
+    ctx.synchronize()
+    m = buf[:, :n]
+    assert bool((buf[:, n:] == -7.0).all())
+    assert bool((m == m.T).all()) and bool((torch.diagonal(m) == 0).all())
+    d = (m.abs().float().view(torch.int32) - flt.abs().view(torch.int32)).abs()
+    assert int(d.max()) <= 1 and int((d == 1).sum()) <= max(2, 1e-6 * n * n)
+    assert mx <= float(m.max())
