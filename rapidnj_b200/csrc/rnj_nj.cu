@@ -27,12 +27,14 @@
 //     (a warp per row; zero of either sign as +0), each candidate is compared
 //     in full with the highest row of its hash group (a warp per pair), and rows
 //     that differ (hash collisions, NaN entries) form new groups;
-//   * each unmarked row is sorted by a CTA: 64-bit items (the distance's bits
-//     made order-preserving, then j) in ascending j, and a stable LSD radix
-//     sort on the distance's four bytes (ranking inside each warp by ballots;
-//     a pass whose digit is the same for the whole row is skipped) gives the
-//     reference's order with equal distances in ascending j; rows of up to
-//     8192 items in shared memory, longer ones in the CTA's global scratch rows.
+//   * each unmarked row is sorted by a CTA: the distances' bits made
+//     order-preserving, items in ascending j, and a stable LSD radix sort
+//     (ranking inside each warp by ballots) gives the reference's order with
+//     equal distances in ascending j.  Rows of up to 16,384 items live in
+//     registers and shared memory, CTAs of 128 to 1,024 threads by length,
+//     and sort on as many bits as their own smallest and largest distance
+//     differ in, nine a pass; longer rows go through the CTA's global
+//     scratch rows, a byte a pass.
 // The O(n) parts (separations, running maximum, the redundancy classes) run on
 // the host from the per-row results.
 #include <cuda_runtime.h>
@@ -53,7 +55,7 @@ namespace {
 
 constexpr int kRowStages = 8;    // 32 x 32 tiles in the ring of a row-pass warp
 constexpr int kTileLd = 33;      // padded tile row: lane l reads bank (l + k) % 32
-constexpr int kSortBlock = 8192; // entries of a row sorted in shared memory
+constexpr int kSortBlock = 8192; // entries of a chunk of a long row
 constexpr int kSortThreads = 1024;
 
 enum : uint32_t { kRowZero = 1u, kRowBadDiag = 4u };
@@ -189,18 +191,191 @@ __device__ __forceinline__ unsigned long long sort_key(float v, int j) {
   return ((unsigned long long)f << 32) | (uint32_t)j;
 }
 
-// Pass 3: a CTA per unmarked row i (rows[], longest first).  The unmarked j < i
-// (rank[j] = unmarked rows below j, rank[i] of them in all) become 64-bit items
-// (order-preserving distance key << 32 | j) in ascending j, and a stable LSD
-// radix sort on the key's four bytes orders them by distance with equal
-// distances in ascending j; the first min(rank[i], cap) are written as
-// (j, matrix[i][j]).  Each pass, chunk by chunk (8192 items: warp w, slot s,
-// lane l holds item w 256 + s 32 + l): a stable rank inside each warp by
-// ballots, the per-(digit, warp) offsets from the digit bases, and the scatter.
-// The digit bases come from the chunk's own counts when the row is one chunk,
-// else from a histogram of the row first; a pass in which one digit holds every
-// item is skipped.  Rows of up to 8192 items live in shared memory, longer ones
-// in the CTA's scratch rows.
+// Pass 3, rows of at most kThreads * kItems unmarked entries: a CTA per row.  kept
+// lists the unmarked rows in ascending order, so entry t of row i is column
+// kept[t], t < rank[i].  Thread (warp w, lane l) holds items w 32 kItems + 32 s + l:
+// the key less the row's smallest, and t.  Per pass of kWidth bits: each warp's
+// digit counts and the rank of every item among the warp's equal digits (peers by
+// ballots, in slot and lane order, so the sort is stable), the counts scanned over
+// the warps and the digits, and the items scattered into the one shared copy (all
+// of them are in registers).  The last pass scatters t alone, and the row is
+// written as (j, matrix[i][j]).
+//
+// Measured over a 10,000 x 10,000 matrix (50 M entries): 1,113 us (by class 440, 499,
+// 123 and 50), against 2,570 us of one 1,024-thread CTA per SM with 64-bit items,
+// four byte-wide passes and rows over 8,192 entries in global memory.  Bound by
+// issue, the ballots first (a ballot and three more instructions a key bit).  Small
+// CTAs let several rows share an SM, so that one's barriers and scans are the others'
+// time to issue: hence classes, and 64 registers a thread (1,024 threads an SM; at 114
+// the 512-thread class had one CTA an SM and took 938 us).  Keys less their minimum
+// need three passes (27 bits are typical) instead of four.
+constexpr int kWidth = 9;  // key bits of a pass
+
+template <int kThreads, int kItems>
+struct BlockSort {
+  static constexpr int kWarps = kThreads / 32, kMax = kThreads * kItems;
+  uint32_t key[kMax];
+  uint16_t idx[kMax];
+  alignas(16) uint16_t cnt[kWarps][1 << kWidth];  // per warp and digit: counts, then offsets
+  uint32_t base[1 << kWidth];
+  uint32_t red[2][kWarps];
+};
+
+// One pass over kWidth bits of the keys from `shift`: counts, ranks, scans,
+// scatter (every thread of the block; ends with a block barrier).
+template <int kThreads, int kItems>
+__device__ __forceinline__ void sort_pass(BlockSort<kThreads, kItems> &S, uint32_t (&x)[kItems],
+                                          uint32_t (&id)[kItems], int cnt, int shift, bool last) {
+  constexpr int kWarps = kThreads / 32, kDigits = 1 << kWidth;
+  constexpr int kPer = kDigits > kThreads ? kDigits / kThreads : 1;  // digits of a thread
+  const int th = threadIdx.x, lane = th & 31, warp = th >> 5;
+  const int w0 = warp * (32 * kItems);  // the warp's first item
+  const uint32_t lt = (1u << lane) - 1u;
+  uint16_t *const mine = S.cnt[warp];
+  // Each warp clears and fills its own counters.
+  for (int k = lane; k < kDigits / 8; k += 32)
+    reinterpret_cast<uint4 *>(mine)[k] = make_uint4(0u, 0u, 0u, 0u);
+  __syncwarp();
+#pragma unroll
+  for (int s = 0; s < kItems; ++s) {
+    if (w0 + 32 * s < cnt) {  // uniform per warp
+      const bool ok = w0 + 32 * s + lane < cnt;
+      const uint32_t d = (x[s] >> shift) & (uint32_t)(kDigits - 1);
+      uint32_t peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+      for (int b = 0; b < kWidth; ++b) {
+        const uint32_t bit = (d >> b) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, bit);
+        peers &= m ^ (bit - 1u);
+      }
+      const uint32_t before = ok ? mine[d] : 0u;
+      __syncwarp();
+      if (ok && (peers & lt) == 0) mine[d] = (uint16_t)(before + __popc(peers));
+      __syncwarp();
+      // (t below 2^16, the rank above it: both are below 2^14)
+      id[s] = (id[s] & 0xFFFFu) | (before + __popc(peers & lt)) << 16;
+    }
+  }
+  __syncthreads();
+  // Counts -> offsets within the digit (over the warps), then the digits' bases.
+  uint32_t sum = 0, first[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; ++k) {
+    const int d = th * kPer + k;
+    first[k] = sum;
+    if (d < kDigits) {
+      uint32_t v[kWarps], run = 0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) v[w] = S.cnt[w][d];
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        S.cnt[w][d] = (uint16_t)run;
+        run += v[w];
+      }
+      sum += run;
+    }
+  }
+  uint32_t incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) S.red[0][warp] = incl;
+  __syncthreads();
+  const uint32_t part = lane < kWarps ? S.red[0][lane] : 0u;
+  const uint32_t ahead = __reduce_add_sync(0xffffffffu, lane < warp ? part : 0u) + incl - sum;
+#pragma unroll
+  for (int k = 0; k < kPer; ++k)
+    if (th * kPer + k < kDigits) S.base[th * kPer + k] = ahead + first[k];
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < kItems; ++s) {
+    if (w0 + 32 * s + lane < cnt) {
+      const uint32_t d = (x[s] >> shift) & (uint32_t)(kDigits - 1);
+      const uint32_t p = S.base[d] + mine[d] + (id[s] >> 16);
+      S.idx[p] = (uint16_t)id[s];
+      if (!last) S.key[p] = x[s];
+    }
+  }
+  __syncthreads();
+}
+
+template <int kThreads, int kItems>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads)
+    nj_sort_block_kernel(const float *__restrict__ M, size_t ld, const int *__restrict__ kept,
+                         const int *__restrict__ rank, const int *__restrict__ rows,
+                         rnj_cluster_pair *__restrict__ out, size_t out_ld, int cap) {
+  constexpr int kWarps = kThreads / 32;
+  extern __shared__ __align__(16) unsigned char nj_block_smem[];
+  BlockSort<kThreads, kItems> &S = *reinterpret_cast<BlockSort<kThreads, kItems> *>(nj_block_smem);
+  const int th = threadIdx.x, lane = th & 31, warp = th >> 5;
+  const int i = rows[blockIdx.x];
+  const int cnt = rank[i];
+  const float *row = M + (size_t)i * ld;
+  const int t0 = warp * (32 * kItems) + lane;
+  uint32_t x[kItems], id[kItems];
+  uint32_t lo = 0xFFFFFFFFu, hi = 0u;
+#pragma unroll
+  for (int s = 0; s < kItems; ++s) {
+    const int t = t0 + 32 * s;
+    id[s] = (uint32_t)t;
+    x[s] = 0xFFFFFFFFu;
+    if (t < cnt) {
+      x[s] = (uint32_t)(sort_key(row[kept[t]], 0) >> 32);
+      lo = min(lo, x[s]);
+      hi = max(hi, x[s]);
+    }
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0) {
+    S.red[0][warp] = lo;
+    S.red[1][warp] = hi;
+  }
+  __syncthreads();
+  lo = __reduce_min_sync(0xffffffffu, S.red[0][lane % kWarps]);
+  hi = __reduce_max_sync(0xffffffffu, S.red[1][lane % kWarps]);
+  __syncthreads();  // (the words are used again)
+  const int bits = max(1, 32 - __clz((int)(hi - lo)));
+  const int passes = (bits + kWidth - 1) / kWidth;
+#pragma unroll
+  for (int s = 0; s < kItems; ++s) x[s] -= lo;
+  for (int pass = 0; pass < passes; ++pass) {
+    const bool last = pass + 1 == passes;
+    sort_pass(S, x, id, cnt, pass * kWidth, last);
+    if (last) break;
+#pragma unroll
+    for (int s = 0; s < kItems; ++s) {
+      const int t = t0 + 32 * s;
+      if (t < cnt) {
+        x[s] = S.key[t];
+        id[s] = S.idx[t];
+      }
+    }
+    // (the next scatter comes after barriers that follow these reads)
+  }
+  const int keepn = cap > 0 ? min(cnt, cap) : cnt;
+  rnj_cluster_pair *o = out + (size_t)i * out_ld;
+  for (int t = th; t < keepn; t += kThreads) {
+    const int j = kept[S.idx[t]];
+    rnj_cluster_pair cp;
+    cp.id = (unsigned int)j;
+    cp.distance = row[j];  // the stored value, -0 kept
+    o[t] = cp;
+  }
+}
+
+// Pass 3 of longer rows: CTAs take the unmarked rows i in turn (rows[], longest
+// first).  The unmarked j < i (rank[j] = unmarked rows below j, rank[i] of them in
+// all) become 64-bit items (order-preserving distance key << 32 | j) in ascending j
+// in the CTA's scratch rows, and a stable LSD radix sort on the key's four bytes
+// orders them by distance with equal distances in ascending j; the first
+// min(rank[i], cap) are written as (j, matrix[i][j]).  Each pass: a histogram of
+// the row's digits gives the digit bases (a pass in which one digit holds every
+// item is skipped), then chunk by chunk (8192 items: warp w, slot s, lane l holds
+// item w 256 + s 32 + l) a stable rank inside each warp by ballots, the
+// per-(digit, warp) offsets from the digit bases, and the scatter.
 constexpr int kRadixDigits = 256;
 constexpr int kWarpsPerSort = kSortThreads / 32;
 constexpr int kItems = kSortBlock / kSortThreads;  // per thread and chunk
@@ -222,8 +397,6 @@ __device__ __forceinline__ uint32_t digit_peers(uint32_t d, bool valid) {
 }
 
 struct SortShared {
-  u64 a[kSortBlock];
-  u64 b[kSortBlock];
   uint32_t wcnt[kWarpsPerSort * kRadixDigits];  // [warp][digit]
   uint32_t dtot[kRadixDigits];
   uint32_t dbase[kRadixDigits];
@@ -272,37 +445,26 @@ __global__ void __launch_bounds__(kSortThreads, 1)
     const int cnt = rank[i];
     if (cnt == 0) continue;  // uniform over the CTA
     const float *row = M + (size_t)i * ld;
-    u64 *A, *B;
-    if (cnt <= kSortBlock) {
-      A = S.a;
-      B = S.b;
-    } else {
-      A = scratch + (size_t)blockIdx.x * 2 * scratch_per_cta;
-      B = A + scratch_per_cta;
-    }
+    u64 *A = scratch + (size_t)blockIdx.x * 2 * scratch_per_cta, *B = A + scratch_per_cta;
     for (int j = th; j < i; j += blockDim.x)
       if (keep[j]) A[rank[j]] = sort_key(row[j], j);
     __syncthreads();
     for (int pass = 0; pass < 4; ++pass) {
       const int shift = 32 + 8 * pass;
-      const bool chunked = cnt > kSortBlock;
-      if (chunked) {
-        // Histogram of the row's digits (warp-aggregated shared atomics); a row
-        // of one chunk takes its totals from the ranking instead.
-        for (int d = th; d < kRadixDigits; d += blockDim.x) S.dtot[d] = 0;
-        __syncthreads();
-        for (int t0 = 0; t0 < cnt; t0 += blockDim.x) {
-          const int t = t0 + th;
-          const bool ok = t < cnt;
-          const uint32_t d = ok ? (uint32_t)((A[t] >> shift) & 255u) : 0u;
-          const uint32_t peers = digit_peers(d, ok);
-          if (ok && (peers & lt) == 0) atomicAdd(&S.dtot[d], (uint32_t)__popc(peers));
-        }
-        __syncthreads();
-        scan_digits(S, cnt, warp, lane);
-        __syncthreads();
-        if (S.skip) continue;  // uniform: every item has the same digit
+      // Histogram of the row's digits (warp-aggregated shared atomics).
+      for (int d = th; d < kRadixDigits; d += blockDim.x) S.dtot[d] = 0;
+      __syncthreads();
+      for (int t0 = 0; t0 < cnt; t0 += blockDim.x) {
+        const int t = t0 + th;
+        const bool ok = t < cnt;
+        const uint32_t d = ok ? (uint32_t)((A[t] >> shift) & 255u) : 0u;
+        const uint32_t peers = digit_peers(d, ok);
+        if (ok && (peers & lt) == 0) atomicAdd(&S.dtot[d], (uint32_t)__popc(peers));
       }
+      __syncthreads();
+      scan_digits(S, cnt, warp, lane);
+      __syncthreads();
+      if (S.skip) continue;  // uniform: every item has the same digit
       for (int c0 = 0; c0 < cnt; c0 += kSortBlock) {
         for (int k = th; k < kWarpsPerSort * kRadixDigits; k += blockDim.x) S.wcnt[k] = 0;
         __syncthreads();
@@ -322,18 +484,6 @@ __global__ void __launch_bounds__(kSortThreads, 1)
           rk[s] = before + __popc(peers & lt);
         }
         __syncthreads();
-        if (!chunked) {
-          // One chunk: digit totals from the warps' counts, then the bases.
-          for (int d = th; d < kRadixDigits; d += blockDim.x) {
-            uint32_t t = 0;
-            for (int w = 0; w < kWarpsPerSort; ++w) t += S.wcnt[w * kRadixDigits + d];
-            S.dtot[d] = t;
-          }
-          __syncthreads();
-          scan_digits(S, cnt, warp, lane);
-          __syncthreads();
-          if (S.skip) break;  // uniform; the pass leaves the items in place
-        }
         // Offsets: digit base, then the warps in order; the base moves on by the
         // chunk's items of that digit.
         for (int d = th; d < kRadixDigits; d += blockDim.x) {
@@ -356,7 +506,6 @@ __global__ void __launch_bounds__(kSortThreads, 1)
         }
         __syncthreads();
       }
-      if (!chunked && S.skip) continue;
       u64 *tmp = A;
       A = B;
       B = tmp;
@@ -559,40 +708,72 @@ extern "C" int rnj_nj_init(rnj_ctx *ctx, const float *d_matrix, int n, size_t ld
     for (int i = 0; i < n; ++i)
       o->row_lengths[i] = keep[i] ? (cap > 0 ? std::min(rank[i], cap) : rank[i]) : 0;
   if (o->sorted && !rows.empty()) {
-    int *d_rank = nullptr, *d_rows = nullptr;
+    std::vector<int> kept;
+    for (int i = 0; i < n; ++i)
+      if (keep[i]) kept.push_back(i);
+    int *d_rank = nullptr, *d_rows = nullptr, *d_kept = nullptr;
     uint8_t *d_keep = nullptr;
     NJ_CUDA(buf.alloc(&d_rank, (size_t)n * sizeof(int)), "nj buffers");
-    NJ_CUDA(buf.alloc(&d_keep, (size_t)n), "nj buffers");
+    NJ_CUDA(buf.alloc(&d_kept, kept.size() * sizeof(int)), "nj buffers");
     NJ_CUDA(buf.alloc(&d_rows, rows.size() * sizeof(int)), "nj buffers");
     NJ_CUDA(cudaMemcpyAsync(d_rank, rank.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, st),
             "nj copy");
-    NJ_CUDA(cudaMemcpyAsync(d_keep, keep.data(), (size_t)n, cudaMemcpyHostToDevice, st), "nj copy");
+    NJ_CUDA(cudaMemcpyAsync(d_kept, kept.data(), kept.size() * sizeof(int), cudaMemcpyHostToDevice,
+                            st),
+            "nj copy");
     NJ_CUDA(cudaMemcpyAsync(d_rows, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice,
                             st),
             "nj copy");
-    const int smem = (int)sizeof(SortShared);
-    NJ_CUDA(cudaFuncSetAttribute(nj_sort_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 smem),
-            "nj sort attribute");
-    int per_sm = 1;
-    NJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nj_sort_rows_kernel, kSortThreads,
-                                                          smem),
-            "nj sort occupancy");
-    const int grid =
-        (int)std::min<size_t>(rows.size(), (size_t)std::max(1, per_sm) * ctx->num_sms);
-    // Rows of more than kSortBlock items: two scratch rows per CTA.
-    const size_t longest = (size_t)rank[rows[0]];
-    u64 *d_scratch = nullptr;
-    size_t per_cta = 0;
-    if (longest > (size_t)kSortBlock) {
-      per_cta = longest;
-      NJ_CUDA(buf.alloc(&d_scratch, (size_t)grid * 2 * per_cta * sizeof(u64)),
-              "nj sort scratch");
+    // The rows, longest first, by the CTA that sorts them: a run of `rows` per kind.
+    size_t at = 0;
+    auto run_of = [&](int most) {  // rows of more than `most` entries from `at` on
+      size_t e = at;
+      while (e < rows.size() && rank[rows[e]] > most) ++e;
+      return e - at;
+    };
+    if (const size_t big = run_of(BlockSort<1024, 16>::kMax)) {
+      NJ_CUDA(buf.alloc(&d_keep, (size_t)n), "nj buffers");
+      NJ_CUDA(cudaMemcpyAsync(d_keep, keep.data(), (size_t)n, cudaMemcpyHostToDevice, st), "nj copy");
+      const int smem = (int)sizeof(SortShared);
+      NJ_CUDA(cudaFuncSetAttribute(nj_sort_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   smem),
+              "nj sort attribute");
+      int per_sm = 1;
+      NJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nj_sort_rows_kernel,
+                                                            kSortThreads, smem),
+              "nj sort occupancy");
+      const int grid = (int)std::min<size_t>(big, (size_t)std::max(1, per_sm) * ctx->num_sms);
+      // Two scratch rows per CTA.
+      const size_t per_cta = (size_t)rank[rows[0]];
+      u64 *d_scratch = nullptr;
+      NJ_CUDA(buf.alloc(&d_scratch, (size_t)grid * 2 * per_cta * sizeof(u64)), "nj sort scratch");
+      nj_sort_rows_kernel<<<grid, kSortThreads, smem, st>>>(d_matrix, ld, d_rank, d_keep, d_rows,
+                                                           (int)big, d_scratch, per_cta, o->sorted,
+                                                           o->sorted_ld, cap);
+      NJ_CUDA(cudaGetLastError(), "nj sort");
+      at += big;
     }
-    nj_sort_rows_kernel<<<grid, kSortThreads, smem, st>>>(d_matrix, ld, d_rank, d_keep, d_rows,
-                                                         (int)rows.size(), d_scratch, per_cta,
-                                                         o->sorted, o->sorted_ld, cap);
-    NJ_CUDA(cudaGetLastError(), "nj sort");
+    auto block_sort = [&](auto kernel, int threads, size_t smem, size_t count) -> cudaError_t {
+      if (count == 0) return cudaSuccess;
+      cudaError_t e =
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      kernel<<<(unsigned)count, threads, smem, st>>>(d_matrix, ld, d_kept, d_rank, d_rows + at,
+                                                     o->sorted, o->sorted_ld, cap);
+      at += count;
+      return cudaGetLastError();
+    };
+    NJ_CUDA(block_sort(nj_sort_block_kernel<1024, 16>, 1024, sizeof(BlockSort<1024, 16>),
+                       run_of(BlockSort<512, 16>::kMax)),
+            "nj sort");
+    NJ_CUDA(block_sort(nj_sort_block_kernel<512, 16>, 512, sizeof(BlockSort<512, 16>),
+                       run_of(BlockSort<256, 16>::kMax)),
+            "nj sort");
+    NJ_CUDA(block_sort(nj_sort_block_kernel<256, 16>, 256, sizeof(BlockSort<256, 16>),
+                       run_of(BlockSort<128, 16>::kMax)),
+            "nj sort");
+    NJ_CUDA(block_sort(nj_sort_block_kernel<128, 16>, 128, sizeof(BlockSort<128, 16>), run_of(0)),
+            "nj sort");
   }
   NJ_CUDA(cudaStreamSynchronize(st), "nj sync");
   return RNJ_OK;

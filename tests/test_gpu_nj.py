@@ -159,3 +159,38 @@ def test_after_distance_call(ctx):
     got["rows"] = device_rows(got)
     compare(got, want, 0, exact_ties=True)
     assert got["redundant_to_master"][10] == 500
+
+
+@pytest.mark.parametrize("kind", ["grid", "equal", "ulps", "bits"])
+@pytest.mark.parametrize("cap", [0, 700])
+def test_row_lengths_around_the_sort_classes(ctx, kind, cap):
+    """Rows either side of every length at which another kernel sorts them, keys that
+    need 1, 10 and 32 bits, and the order of equal, infinite and NaN keys: exactly the
+    stable order of the order-preserving bits."""
+    n = 16388
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    if kind == "grid":
+        m, _ = points_matrix(n, 3, dup=0.0)
+        m = m + 0.25
+    elif kind == "equal":
+        m = torch.ones((n, n), device="cuda")
+    elif kind == "ulps":  # keys 0..512 less their minimum: one bit more than a pass takes
+        k = torch.randint(0, 513, (n, n), device="cuda", generator=gen, dtype=torch.int32)
+        m = (k + 0x3F800000).view(torch.float32)
+    else:  # any non-zero bits: both signs, infinities, NaN
+        k = torch.randint(1, 2**31 - 1, (n, n), device="cuda", generator=gen, dtype=torch.int32)
+        k[:, ::3] += -2**31
+        k[:, 1::41] = 0x7F800000
+        m = k.view(torch.float32)
+    m.fill_diagonal_(0.0)
+    got = ctx.nj_init(m, cap=cap)
+    rows = sorted({r for e in (1, 32, 512, 2048, 4096, 8192, 16384) for r in (e - 1, e, e + 1)} | {n - 1})
+    for i in rows:
+        b = m[i, :i].cpu().numpy().view(np.uint32).astype(np.int64)
+        key = np.where(b >> 31, 0xFFFFFFFF - b, b + 0x80000000)
+        order = np.argsort(key, kind="stable")
+        order = order[:cap] if cap else order
+        assert got["row_lengths"][i] == len(order)
+        s = got["sorted"][i, :len(order)].cpu().numpy()
+        assert np.array_equal(s[:, 0], order), i
+        assert np.array_equal(s[:, 1].view(np.uint32), b[order].astype(np.uint32)), i
