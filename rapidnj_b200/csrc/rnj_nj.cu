@@ -14,8 +14,8 @@
 //      rapidNJMem (rapidNJMem.cpp:138-153).
 //
 // On the device:
-//   * one pass reads the matrix once: a warp owns 32 rows and streams them in
-//     32 x 32 tiles (cp.async into shared memory, eight tiles in its ring), then
+//   * one pass reads the matrix once: a warp owns 32 rows and other warps stream
+//     them in 32 x 64 tiles (cp.async into shared memory, six tiles in the ring);
 //     every lane walks its own row of the tile in column order, so each row is
 //     summed exactly in the reference's order; the same walk counts the row's
 //     zeros (a second zero besides the diagonal is the zero scan of
@@ -53,8 +53,10 @@ using namespace rnj;
 
 namespace {
 
-constexpr int kRowStages = 8;    // 32 x 32 tiles in the ring of a row-pass warp
-constexpr int kTileLd = 33;      // padded tile row: lane l reads bank (l + k) % 32
+constexpr int kRowCols = 64;     // columns of a row-pass tile of 32 rows
+constexpr int kRowStages = 6;    // tiles in the ring of a row-pass CTA
+constexpr int kRowWarps = 5;     // its warps: one sums, the others fetch
+constexpr int kTileLd = kRowCols + 4;  // padded tile row: 16-byte reads by 8 lanes meet no bank twice
 constexpr int kSortBlock = 8192; // entries of a chunk of a long row
 constexpr int kSortThreads = 1024;
 
@@ -66,6 +68,11 @@ __device__ __forceinline__ void cp_async4(float *smem, const float *gmem, bool v
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void cp_async16(float *smem, const float *gmem, int bytes) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes)
+               : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
@@ -75,27 +82,48 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // Pass 1: per row the float sum in column order, whether it holds a zero off
-// the diagonal, and whether its diagonal entry is non-zero.  A CTA (one warp)
-// owns rows [32 b, 32 b + 32); lane l sums row 32 b + l.  Tile t holds columns
-// [32 t, 32 t + 32) of the 32 rows, in stage t % kRowStages of the ring.  Per
-// entry the lane does no more than the sum needs (a load, the add, a zero
-// test), so that the pass runs at the rate the matrix streams in.
-__global__ void __launch_bounds__(32)
+// the diagonal, and whether its diagonal entry is non-zero.  A CTA owns rows
+// [32 b, 32 b + 32); lane l of warp 0 sums row 32 b + l.  Tile t holds columns
+// from kRowCols t on of the 32 rows, in stage t % kRowStages of the ring, fetched by
+// the other warps, eight rows each.  The sums are a serial chain per row and the
+// matrix has few warps' worth of rows, so warp 0 does nothing else.  10,000 x 10,000
+// (60 us of reading): 114 us; 275 with one warp that fetches 4-byte pieces and sums,
+// 157 with the fetching moved to other warps, 130 with 16-byte copies, 114 with 64
+// columns a tile in place of 32.  What is left is the chain and a barrier a tile.
+// kVec: the rows start on 16-byte boundaries (base and ld), so a copy is 16 bytes.
+template <bool kVec>
+__global__ void __launch_bounds__(32 * kRowWarps)
     nj_row_pass_kernel(const float *__restrict__ M, int n, size_t ld, float *__restrict__ sums,
                        uint32_t *__restrict__ flags) {
-  extern __shared__ float tiles[];  // [kRowStages][32 * kTileLd]
-  const int lane = threadIdx.x;
+  extern __shared__ __align__(16) float tiles[];  // [kRowStages][32 * kTileLd]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row0 = blockIdx.x * 32;
-  const int ntile = (n + 31) / 32;
+  const int ntile = (n + kRowCols - 1) / kRowCols;
   auto issue = [&](int t) {
-    if (t < ntile) {
+    if (t < ntile && warp > 0) {
+      constexpr int kRows = 32 / (kRowWarps - 1);
+      const int r0 = (warp - 1) * kRows;
       float *dst = tiles + (t % kRowStages) * (32 * kTileLd);
-      const int c = t * 32 + lane;
-#pragma unroll 8
-      for (int r = 0; r < 32; ++r) {
-        const int row = row0 + r;
-        const bool ok = row < n && c < n;
-        cp_async4(dst + r * kTileLd + lane, ok ? M + (size_t)row * ld + c : M, ok);
+      if (kVec) {
+        constexpr int kQuads = kRowCols / 4;  // 16-byte pieces of a tile row
+        const int k = 4 * (lane % kQuads), c = t * kRowCols + k;
+#pragma unroll
+        for (int q = 0; q < kRows; q += 32 / kQuads) {
+          const int r = r0 + q + lane / kQuads, row = row0 + r;
+          const int cols = row < n ? min(max(n - c, 0), 4) : 0;
+          cp_async16(dst + r * kTileLd + k, cols > 0 ? M + (size_t)row * ld + c : M, 4 * cols);
+        }
+      } else {
+#pragma unroll
+        for (int r = r0; r < r0 + kRows; ++r) {
+          const int row = row0 + r;
+#pragma unroll
+          for (int k = lane; k < kRowCols; k += 32) {
+            const int c = t * kRowCols + k;
+            const bool ok = row < n && c < n;
+            cp_async4(dst + r * kTileLd + k, ok ? M + (size_t)row * ld + c : M, ok);
+          }
+        }
       }
     }
     cp_async_commit();  // an empty group past the end keeps the count uniform
@@ -106,28 +134,31 @@ __global__ void __launch_bounds__(32)
   float sum = 0.0f;
   int zeros = 0;
   for (int t = 0; t < ntile; ++t) {
-    issue(t + kRowStages - 1);
-    cp_async_wait<kRowStages - 1>();  // this lane's copies of tile t are done
-    __syncwarp();                     // and every lane's are visible
+    cp_async_wait<kRowStages - 2>();  // this thread's copies of tile t are done,
+    __syncthreads();                  // every thread's are visible, and tile t - 1 is summed:
+    issue(t + kRowStages - 1);        // its stage is refilled
+    if (warp > 0) continue;
     const float *row = tiles + (t % kRowStages) * (32 * kTileLd) + lane * kTileLd;
-    if (t * 32 + 32 <= n) {
+    if ((t + 1) * kRowCols <= n) {
 #pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        const float v = row[k];
-        sum += v;
-        zeros += v == 0.0f;
+      for (int k = 0; k < kRowCols; k += 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(row + k);
+        sum += v.x;
+        sum += v.y;
+        sum += v.z;
+        sum += v.w;
+        zeros += (v.x == 0.0f) + (v.y == 0.0f) + (v.z == 0.0f) + (v.w == 0.0f);
       }
     } else {
-      for (int k = 0; k < n - t * 32; ++k) {
+      for (int k = 0; k < n - t * kRowCols; ++k) {
         const float v = row[k];
         sum += v;
         zeros += v == 0.0f;
       }
     }
-    __syncwarp();  // the stage is refilled by the next iteration's issue
   }
   cp_async_wait<0>();
-  if (my_row < n) {
+  if (warp == 0 && my_row < n) {
     const float diag = M[(size_t)my_row * ld + my_row];
     sums[my_row] = sum;
     // with a zero diagonal, a second zero is one off the diagonal
@@ -566,10 +597,11 @@ extern "C" int rnj_nj_init(rnj_ctx *ctx, const float *d_matrix, int n, size_t ld
   NJ_CUDA(buf.alloc(&d_sums, (size_t)n * sizeof(float)), "nj buffers");
   NJ_CUDA(buf.alloc(&d_flags, (size_t)n * sizeof(uint32_t)), "nj buffers");
   const int row_smem = kRowStages * 32 * kTileLd * (int)sizeof(float);
-  NJ_CUDA(cudaFuncSetAttribute(nj_row_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               row_smem),
+  const bool vec = ((uintptr_t)d_matrix & 15) == 0 && ld % 4 == 0;
+  auto *row_pass = vec ? nj_row_pass_kernel<true> : nj_row_pass_kernel<false>;
+  NJ_CUDA(cudaFuncSetAttribute(row_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, row_smem),
           "nj row pass attribute");
-  nj_row_pass_kernel<<<(n + 31) / 32, 32, row_smem, st>>>(d_matrix, n, ld, d_sums, d_flags);
+  row_pass<<<(n + 31) / 32, 32 * kRowWarps, row_smem, st>>>(d_matrix, n, ld, d_sums, d_flags);
   NJ_CUDA(cudaGetLastError(), "nj row pass");
   std::vector<float> sums(n);
   std::vector<uint32_t> flags(n);

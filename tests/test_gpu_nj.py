@@ -194,3 +194,17 @@ def test_row_lengths_around_the_sort_classes(ctx, kind, cap):
         s = got["sorted"][i, :len(order)].cpu().numpy()
         assert np.array_equal(s[:, 0], order), i
         assert np.array_equal(s[:, 1].view(np.uint32), b[order].astype(np.uint32)), i
+
+
+@pytest.mark.parametrize("n", [1, 3, 63, 64, 65, 129, 450])
+@pytest.mark.parametrize("align", [True, False])
+def test_row_sums_in_column_order_at_tile_edges(ctx, n, align):
+    """The sums of both copy widths (16 bytes where every row starts on a 16-byte
+    boundary) over ragged tiles: float, column by column, nothing past column n."""
+    ld = (n + 3) // 4 * 4 + (4 if align else 5)
+    x = np.random.default_rng(n).random((n, n)).astype(np.float32) + np.float32(0.5)
+    np.fill_diagonal(x, 0.0)
+    got = run(ctx, x, 0, ld - n)
+    want = np.add.accumulate(x, axis=1, dtype=np.float32)[:, -1]
+    assert np.array_equal(got["sums"], want)
+    assert not got["possible_redundant"].any()
