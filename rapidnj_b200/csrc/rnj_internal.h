@@ -179,7 +179,10 @@ struct alignas(16) PackJob {
 cudaError_t launch_pack_chars(const uint8_t *d_chars, size_t ld, const Packed &p,
                               const uint8_t lut[256], cudaStream_t s);
 cudaError_t launch_presence(const uint8_t *d_chars, size_t ld, int n, int L,
-                            uint32_t *d_mask /*8 words*/, cudaStream_t s);
+                            uint32_t *d_mask /*8 words*/, cudaStream_t s,
+                            uint32_t *h_report = nullptr);
+// (h_report: page-locked, 8 words, filled with the mask; d_mask then has 9 words,
+// zero before the launch and after it.)
 // Row segment of a presence-scan work unit (one warp), bytes.
 constexpr int kPresenceSeg = 4096;
 // Many alignments in one launch each.  Presence: units = sum of

@@ -199,9 +199,13 @@ __device__ __forceinline__ void flush_flags(uint8_t *flags, uint32_t *mask, int 
   __syncwarp();
 }
 
+// report: null, or page-locked host words that the last CTA fills with the whole
+// mask, leaving mask[0 .. 8) and the count of finished CTAs in mask[8] zero for
+// the next call (they are zero before the first one).
 __global__ void __launch_bounds__(256) presence_kernel(const uint8_t *__restrict__ chars,
                                                        size_t ld, int n, int L,
-                                                       uint32_t *__restrict__ mask) {
+                                                       uint32_t *__restrict__ mask,
+                                                       volatile uint32_t *report) {
   __shared__ __align__(16) uint8_t s_flags[kPresenceWarps][256];
   const int lane = threadIdx.x & 31;
   uint8_t *flags = s_flags[threadIdx.x >> 5];
@@ -217,6 +221,17 @@ __global__ void __launch_bounds__(256) presence_kernel(const uint8_t *__restrict
     mark_span(chars + (size_t)i * ld + k0, min(L - k0, kPresenceSeg), flags, lane);
   }
   flush_flags(flags, mask, lane);
+  if (!report) return;
+  __shared__ bool s_last;
+  __threadfence();  // this thread's ORs before its CTA is counted
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&mask[8], 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (s_last) {
+    __threadfence();
+    if (threadIdx.x < 8) report[threadIdx.x] = atomicExch(&mask[threadIdx.x], 0u);
+    if (threadIdx.x == 8) atomicExch(&mask[8], 0u);
+  }
 }
 
 // Presence masks of many alignments: a warp per row segment of any job, its
@@ -844,9 +859,9 @@ cudaError_t launch_pack_chars(const uint8_t *d_chars, size_t ld, const Packed &p
 }
 
 cudaError_t launch_presence(const uint8_t *d_chars, size_t ld, int n, int L, uint32_t *d_mask,
-                            cudaStream_t s) {
+                            cudaStream_t s, uint32_t *h_report) {
   const long long units = (long long)n * ((L + kPresenceSeg - 1) / kPresenceSeg);  // a warp each
-  presence_kernel<<<grid_for(units * 32, 256), 256, 0, s>>>(d_chars, ld, n, L, d_mask);
+  presence_kernel<<<grid_for(units * 32, 256), 256, 0, s>>>(d_chars, ld, n, L, d_mask, h_report);
   return cudaGetLastError();
 }
 

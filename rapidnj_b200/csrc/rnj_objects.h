@@ -33,7 +33,7 @@ struct rnj_ctx {
   cudaStream_t stream = nullptr;
   int num_sms = 148;
   rnj::Scratch scratch;
-  uint32_t *d_mask = nullptr;             // presence mask (8 words)
+  uint32_t *d_mask = nullptr;             // presence_mask's: 8 words and a count, zero between calls
   uint32_t *h_mask = nullptr;             // pinned
   int *h_max = nullptr;                   // pinned max bits / error word
   // Device error word of the single-alignment calls (bit 0: a bounded wait ran
@@ -59,6 +59,8 @@ struct rnj_ctx {
   size_t h_file_cap = 0;
 };
 
+// The byte-presence mask of an alignment into ctx->h_mask (synchronises the stream; rnj_api.cu).
+int presence_mask(rnj_ctx *ctx, const uint8_t *d_chars, int n, int L, size_t ld);
 // Grows the context's packed-count buffer to `tiles` tiles (rnj_api.cu).
 int ensure_packed(rnj_ctx *ctx, long long tiles);
 // Counts + transform of work items [0, nitems) of the tensor-core path in

@@ -238,12 +238,7 @@ int distance_host_streamed(rnj_ctx *ctx, const char *chars, int n, int L, size_t
       RNJ_TRY(cudaMemcpy2DAsync(buf.chars, (size_t)L, chars, ld, (size_t)L, (size_t)n,
                                 cudaMemcpyHostToDevice, ctx->stream),
               "alignment upload");
-    RNJ_TRY(cudaMemsetAsync(ctx->d_mask, 0, 8 * sizeof(uint32_t), ctx->stream), "mask clear");
-    RNJ_TRY(launch_presence(buf.chars, (size_t)L, n, L, ctx->d_mask, ctx->stream), "presence kernel");
-    RNJ_TRY(cudaMemcpyAsync(ctx->h_mask, ctx->d_mask, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                            ctx->stream),
-            "mask copy");
-    RNJ_TRY(cudaStreamSynchronize(ctx->stream), "mask sync");
+    if (const int rc = presence_mask(ctx, buf.chars, n, L, (size_t)L)) return rc;
     int kind = 0;
     lut_for(RNJ_PROTEIN, flags, ctx->h_mask, lut, &kind);
     int ranks = 0;

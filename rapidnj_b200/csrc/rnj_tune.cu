@@ -271,6 +271,9 @@ bool more_reps(const std::vector<float> &t, int reps) {
 int time_plain(rnj_ctx *ctx, TuneBuffers &b, int n, int L, int type, int flags, int model,
                const rnj_tune_params &p, int reps, float *ms) {
   rnj_tune_set(n, L, type, flags, &p);
+  // A -f bucket's choices are those of the bit planes, which its calls take when
+  // the letters need them: they are what is timed.
+  if (type == RNJ_DNA && !(flags & RNJ_FASTDIST)) flags |= RNJ_POPCOUNT;
   std::vector<float> t;
   for (int r = -1; r < 0 || more_reps(t, reps); ++r) {
     if (cudaEventRecord(b.ev[0], ctx->stream) != cudaSuccess) return cuda_error(cudaGetLastError(), "event");

@@ -412,3 +412,43 @@ def test_tensor_core_matches_popcount_kernel(ctx):
         a, am = gpu_matrix(ctx, seqs, oracle.DNA, model, popcount=True)
         b, bm = gpu_matrix(ctx, seqs, oracle.DNA, model)
         assert np.array_equal(a, b) and am == bm
+
+
+NAIVE_LETTERS = ["upper", "upper-ambiguous", "lower", "mixed", "one-a", "one-t", "one-u", "one-U",
+                 "every-byte"]
+
+
+@pytest.mark.parametrize("letters", NAIVE_LETTERS)
+@pytest.mark.parametrize("n,L,pad", [(70, 1536, 0), (129, 1601, 3), (2560, 17, 0), (2, 1537, 1)])
+def test_naive_rules_agree_on_every_layout(ctx, letters, n, L, pad):
+    """The naive rules over alignments whose letters may send them to the fast rules'
+    kernels: counts, distances and double-precision distances equal those of the bit
+    planes (popcount keeps those), the counts also the oracle's."""
+    rng = np.random.default_rng(n + L)
+    seqs = rng.choice(np.frombuffer(b"ACGT-", np.uint8), (n, L), p=[.3, .2, .2, .2, .1])
+    if letters == "upper-ambiguous":
+        extra = rng.choice(np.frombuffer(b"NRYKMSWBDHVnx.?*\x00\xff", np.uint8), (n, L))
+        seqs = np.where(rng.random((n, L)) < 0.1, extra, seqs)
+    elif letters == "lower":
+        seqs = np.char.lower(seqs.view("S1")).view(np.uint8)
+    elif letters == "mixed":
+        low = np.char.lower(seqs.view("S1")).view(np.uint8)
+        seqs = np.where(rng.random((n, L)) < 0.3, low, seqs)
+    elif letters.startswith("one-"):
+        seqs[n - 1, L - 1] = ord(letters[-1])
+    elif letters == "every-byte":
+        seqs = rng.integers(0, 256, (n, L)).astype(np.uint8)
+    buf = torch.zeros((n, L + pad), dtype=torch.uint8, device="cuda")
+    buf[:, :L] = torch.from_numpy(np.ascontiguousarray(seqs))
+    dev = buf[:, :L]
+    planes = gpu_counts(ctx, dev, oracle.DNA, fastdist=False, popcount=True)
+    assert np.array_equal(gpu_counts(ctx, dev, oracle.DNA, fastdist=False), planes)
+    assert np.array_equal(planes[:130, :130], oracle.counts(seqs[:130], oracle.DNA, naive=True))
+    for model in ("jc", "kim"):
+        got, gmax = gpu_matrix(ctx, dev, oracle.DNA, model, fastdist=False)
+        want, wmax = gpu_matrix(ctx, dev, oracle.DNA, model, fastdist=False, popcount=True)
+        assert np.array_equal(got.view(np.uint32), want.view(np.uint32)) and gmax == wmax
+        d = [ctx.distance_f64(ctx.alignment(dev, "dna", fastdist=False, popcount=pc), model)
+             for pc in (False, True)]
+        assert torch.equal(d[0][0].view(torch.int64), d[1][0].view(torch.int64))
+        assert d[0][1] == d[1][1]
