@@ -102,82 +102,9 @@ void free_batch(rnj_batch *b) {
 
 }  // namespace
 
-extern "C" {
-
-int rnj_batch_create(rnj_ctx *ctx, int max_alignments, long long max_tiles, rnj_batch **out) {
-  if (!ctx || !out || max_alignments <= 0 || max_tiles <= 0)
-    return set_error(RNJ_ERR_INVALID, "invalid batch capacity");
-  DeviceGuard g(ctx->device);
-  rnj_batch *b = new rnj_batch();
-  b->ctx = ctx;
-  b->cap_aln = max_alignments;
-  b->cap_tiles = max_tiles;
-  cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_ready, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_uploaded, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_done, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_descs, sizeof(AlnDesc) * max_alignments);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_items_tc, sizeof(WorkItem) * max_tiles);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_items_pc, sizeof(WorkItem) * max_tiles);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_ints, 4 * sizeof(int));
-  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_max, sizeof(int) * max_alignments);
-  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_flags, sizeof(int) * max_tiles);
-  if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_descs, sizeof(AlnDesc) * max_alignments);
-  if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_items_tc, sizeof(WorkItem) * max_tiles);
-  if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_items_pc, sizeof(WorkItem) * max_tiles);
-  if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_ints, 4 * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(b->d_ints, 0, 4 * sizeof(int));
-  if (e != cudaSuccess) {
-    free_batch(b);
-    return cuda_error(e, "batch allocation");
-  }
-  *out = b;
-  return RNJ_OK;
-}
-
-int rnj_batch_add(rnj_batch *b, rnj_aln *aln, int model, float *d_out, size_t ld, int *slot) {
-  if (!b || !aln) return set_error(RNJ_ERR_INVALID, "null argument");
-  if (model != RNJ_JC && model != RNJ_KIMURA) return set_error(RNJ_ERR_INVALID, "unknown model");
-  if (aln->ctx != b->ctx) return set_error(RNJ_ERR_INVALID, "alignment from another context");
-  const Packed &p = aln->p;
-  if (p.n < 1) return set_error(RNJ_ERR_INVALID, "empty alignment");
-  if (!is_tc_kind(p.kind) && p.Wp / kKW > kMaxFusedWords / kKW)
-    return set_error(RNJ_ERR_INVALID, "alignments longer than 65280 columns on the bit-plane "
-                                      "kernels are not batched; use rnj_distance");
-  if (is_tc_kind(p.kind) && p.L > kMaxFusedColumns)
-    return set_error(RNJ_ERR_INVALID, "alignments longer than 65535 columns on the tensor "
-                                      "cores are not batched; use rnj_distance");
-  if ((int)b->entries.size() >= b->cap_aln)
-    return set_error(RNJ_ERR_BUSY, "batch is full (alignments)");
-  const int nt = tiles_of(p.n);
-  const long long ntiles = (p.kind == KIND_NAIVE && (p.flags & RNJ_FULL_ROWS))
-                               ? (long long)nt * nt
-                               : tri_tiles(nt);
-  if (b->tiles_used + ntiles > b->cap_tiles) return set_error(RNJ_ERR_BUSY, "batch is full (tiles)");
-  DeviceGuard g(b->ctx->device);
-  Entry en;
-  en.aln = aln;
-  en.model = model;
-  en.owned = (d_out == nullptr);
-  en.ld = d_out ? ld : (size_t)std::max(4, (p.n + 3) / 4 * 4);
-  en.out = d_out;
-  if (d_out && ld < (size_t)p.n) return set_error(RNJ_ERR_INVALID, "ld < n");
-  if (!d_out) {
-    cudaError_t e = cudaMallocAsync((void **)&en.out, en.ld * p.n * sizeof(float), b->ctx->stream);
-    if (e != cudaSuccess) return cuda_error(e, "batch output allocation");
-  }
-  en.owns_aln = false;
-  en.flag_off = b->tiles_used;
-  en.ntiles = ntiles;
-  b->tiles_used += ntiles;
-  b->entries.push_back(en);
-  if (slot) *slot = (int)b->entries.size() - 1;
-  return RNJ_OK;
-}
-
-int rnj_batch_add_many(rnj_batch *b, int count, const void *const *d_chars, const int *n,
-                       const int *L, const size_t *ld, const int *type, const int *model, int flags,
-                       float *const *d_out, const size_t *ld_out, int *slots) {
+int batch_add_many(rnj_batch *b, int count, const void *const *d_chars, const int *n, const int *L,
+                   const size_t *ld, const int *type, const int *model, int flags,
+                   float *const *d_out, const size_t *ld_out, int *slots, const int *d_cols) {
   if (!b || count < 0 || (count > 0 && (!d_chars || !n || !L || !ld || !type || !model)))
     return set_error(RNJ_ERR_INVALID, "null argument");
   rnj_ctx *ctx = b->ctx;
@@ -294,7 +221,18 @@ int rnj_batch_add_many(rnj_batch *b, int count, const void *const *d_chars, cons
       }
     }
   }
-  {
+  if (d_cols) {
+    // equal shapes: the arena is one array of their features
+    const Packed &p = alns[0]->p;
+    e = !planes.empty() ? cudaErrorInvalidValue
+                        : launch_pack_gathered((const uint8_t *)d_chars[0], ld[0], n[0], L[0], p.Np,
+                                               p.Lk, d_cols, count,
+                                               count > 1 ? offs[1] : 0, arena, ctx->stream);
+    if (e != cudaSuccess) {
+      drop(arena);
+      return cuda_error(e, "gathered pack kernel");
+    }
+  } else {
     const size_t pb = planes.size() * sizeof(PackJob), fb = feats.size() * sizeof(PackJob);
     uint8_t *d_jobs = nullptr;
     e = cudaMallocAsync((void **)&d_jobs, std::max<size_t>(pb + fb, 16), ctx->stream);
@@ -337,6 +275,86 @@ int rnj_batch_add_many(rnj_batch *b, int count, const void *const *d_chars, cons
     if (slots) slots[k] = slot;
   }
   return RNJ_OK;
+}
+
+extern "C" {
+
+int rnj_batch_create(rnj_ctx *ctx, int max_alignments, long long max_tiles, rnj_batch **out) {
+  if (!ctx || !out || max_alignments <= 0 || max_tiles <= 0)
+    return set_error(RNJ_ERR_INVALID, "invalid batch capacity");
+  DeviceGuard g(ctx->device);
+  rnj_batch *b = new rnj_batch();
+  b->ctx = ctx;
+  b->cap_aln = max_alignments;
+  b->cap_tiles = max_tiles;
+  cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_ready, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_uploaded, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_done, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_descs, sizeof(AlnDesc) * max_alignments);
+  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_items_tc, sizeof(WorkItem) * max_tiles);
+  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_items_pc, sizeof(WorkItem) * max_tiles);
+  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_ints, 4 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_max, sizeof(int) * max_alignments);
+  if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_flags, sizeof(int) * max_tiles);
+  if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_descs, sizeof(AlnDesc) * max_alignments);
+  if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_items_tc, sizeof(WorkItem) * max_tiles);
+  if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_items_pc, sizeof(WorkItem) * max_tiles);
+  if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_ints, 4 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemset(b->d_ints, 0, 4 * sizeof(int));
+  if (e != cudaSuccess) {
+    free_batch(b);
+    return cuda_error(e, "batch allocation");
+  }
+  *out = b;
+  return RNJ_OK;
+}
+
+int rnj_batch_add(rnj_batch *b, rnj_aln *aln, int model, float *d_out, size_t ld, int *slot) {
+  if (!b || !aln) return set_error(RNJ_ERR_INVALID, "null argument");
+  if (model != RNJ_JC && model != RNJ_KIMURA) return set_error(RNJ_ERR_INVALID, "unknown model");
+  if (aln->ctx != b->ctx) return set_error(RNJ_ERR_INVALID, "alignment from another context");
+  const Packed &p = aln->p;
+  if (p.n < 1) return set_error(RNJ_ERR_INVALID, "empty alignment");
+  if (!is_tc_kind(p.kind) && p.Wp / kKW > kMaxFusedWords / kKW)
+    return set_error(RNJ_ERR_INVALID, "alignments longer than 65280 columns on the bit-plane "
+                                      "kernels are not batched; use rnj_distance");
+  if (is_tc_kind(p.kind) && p.L > kMaxFusedColumns)
+    return set_error(RNJ_ERR_INVALID, "alignments longer than 65535 columns on the tensor "
+                                      "cores are not batched; use rnj_distance");
+  if ((int)b->entries.size() >= b->cap_aln)
+    return set_error(RNJ_ERR_BUSY, "batch is full (alignments)");
+  const int nt = tiles_of(p.n);
+  const long long ntiles = (p.kind == KIND_NAIVE && (p.flags & RNJ_FULL_ROWS))
+                               ? (long long)nt * nt
+                               : tri_tiles(nt);
+  if (b->tiles_used + ntiles > b->cap_tiles) return set_error(RNJ_ERR_BUSY, "batch is full (tiles)");
+  DeviceGuard g(b->ctx->device);
+  Entry en;
+  en.aln = aln;
+  en.model = model;
+  en.owned = (d_out == nullptr);
+  en.ld = d_out ? ld : (size_t)std::max(4, (p.n + 3) / 4 * 4);
+  en.out = d_out;
+  if (d_out && ld < (size_t)p.n) return set_error(RNJ_ERR_INVALID, "ld < n");
+  if (!d_out) {
+    cudaError_t e = cudaMallocAsync((void **)&en.out, en.ld * p.n * sizeof(float), b->ctx->stream);
+    if (e != cudaSuccess) return cuda_error(e, "batch output allocation");
+  }
+  en.owns_aln = false;
+  en.flag_off = b->tiles_used;
+  en.ntiles = ntiles;
+  b->tiles_used += ntiles;
+  b->entries.push_back(en);
+  if (slot) *slot = (int)b->entries.size() - 1;
+  return RNJ_OK;
+}
+
+int rnj_batch_add_many(rnj_batch *b, int count, const void *const *d_chars, const int *n,
+                       const int *L, const size_t *ld, const int *type, const int *model, int flags,
+                       float *const *d_out, const size_t *ld_out, int *slots) {
+  return batch_add_many(b, count, d_chars, n, L, ld, type, model, flags, d_out, ld_out, slots,
+                        nullptr);
 }
 
 int rnj_batch_run(rnj_batch *b) {

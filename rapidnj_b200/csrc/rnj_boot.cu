@@ -3,10 +3,12 @@
 // rapidNJ's bootstrap (main.cpp:519-532) re-runs the whole distance computation
 // once per replicate on an alignment whose column k is column rand() % L of the
 // original (dataloader::sample_fast_dist, dataloader.cpp:16-58).  Here the
-// original bytes stay on the device: a gather kernel writes the replicates'
-// bytes (column k of replicate r = column cols[r * L + k]), and the replicates
-// of a chunk are packed and counted together as one batch (one presence scan,
-// one pack launch per layout, one persistent launch per kernel family).  The
+// original bytes stay on the device, column k of replicate r being column
+// cols[r * L + k], and the replicates of a chunk are packed and counted together as
+// one batch (one presence scan, one pack launch per layout, one persistent launch
+// per kernel family).  DNA on the tensor cores is packed straight from the original
+// (pack_gathered_kernel); for the other layouts a gather kernel writes the
+// replicates' bytes first.  The
 // caller draws the columns, so the replicates are exactly rapidNJ's when it
 // draws them with the same rand() sequence.
 #include <cuda_runtime.h>
@@ -24,6 +26,7 @@ using namespace rnj;
 
 namespace {
 
+// For the layouts that are packed from bytes:
 // out[r][i][k] = chars[i][cols[r][k]] for replicates r0 .. r0 + nr - 1: a
 // thread per (replicate, row, 4 columns); the column indices are read once per
 // row from L1/L2, the source row is gathered byte by byte, the output written
@@ -65,8 +68,9 @@ extern "C" int rnj_bootstrap(rnj_ctx *ctx, const void *d_chars, int n, int L, si
   if (type != RNJ_DNA && type != RNJ_PROTEIN)
     return set_error(RNJ_ERR_INVALID, "type must be RNJ_DNA or RNJ_PROTEIN");
   if (model != RNJ_JC && model != RNJ_KIMURA) return set_error(RNJ_ERR_INVALID, "unknown model");
-  for (long long k = 0; k < (long long)R * L; ++k)
-    if (cols[k] < 0 || cols[k] >= L) return set_error(RNJ_ERR_INVALID, "column index out of range");
+  bool outside = false;  // (no early exit: the compiler takes many at a time)
+  for (long long k = 0; k < (long long)R * L; ++k) outside |= (unsigned)cols[k] >= (unsigned)L;
+  if (outside) return set_error(RNJ_ERR_INVALID, "column index out of range");
   for (int r = 0; r < R; ++r)
     if (!d_out[r]) return set_error(RNJ_ERR_INVALID, "null output matrix");
   if (R == 0) return RNJ_OK;
@@ -92,29 +96,43 @@ extern "C" int rnj_bootstrap(rnj_ctx *ctx, const void *d_chars, int n, int L, si
     ctx->boot_tiles = (long long)chunk * rep_tiles;
   }
   rnj_batch *b = ctx->boot;
+  // DNA on the tensor cores: the pack gathers the columns itself, and the
+  // replicates' bytes are never written.
+  bool gathered = false;
+  if (type == RNJ_DNA && L <= kMaxGatherColumns) {
+    uint8_t lut[256];
+    int kind = 0;
+    Packed p;
+    lut_for(type, flags, nullptr, lut, &kind);
+    packed_layout(p, n, L, type, flags, kind, lut, false);
+    gathered = p.kind == KIND_DNA_TC;
+  }
   uint8_t *d_rep = nullptr;
   int *d_cols = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&d_rep, (size_t)chunk * rep_bytes, ctx->stream);
+  cudaError_t e = cudaSuccess;
+  if (!gathered) e = cudaMallocAsync((void **)&d_rep, (size_t)chunk * rep_bytes, ctx->stream);
   if (e == cudaSuccess)
     e = cudaMallocAsync((void **)&d_cols, (size_t)chunk * L * sizeof(int), ctx->stream);
   std::vector<const void *> ptrs(chunk);
   std::vector<int> ns(chunk, n), Ls(chunk, L), types(chunk, type), models(chunk, model);
-  std::vector<size_t> lds(chunk, (size_t)L), ldo(chunk, ld_out);
+  std::vector<size_t> lds(chunk, gathered ? ld : (size_t)L), ldo(chunk, ld_out);
   std::vector<int> slots(chunk);
   for (int r0 = 0; r0 < R && e == cudaSuccess && rc == RNJ_OK; r0 += chunk) {
     const int nr = std::min(chunk, R - r0);
     e = cudaMemcpyAsync(d_cols, cols + (size_t)r0 * L, (size_t)nr * L * sizeof(int),
                         cudaMemcpyHostToDevice, ctx->stream);
     if (e != cudaSuccess) break;
-    const long long work = (long long)nr * n * ((L + 3) / 4);
-    long long g = std::min<long long>((work + 255) / 256, 148LL * 32);
-    gather_columns_kernel<<<(unsigned)std::max<long long>(g, 1), 256, 0, ctx->stream>>>(
-        (const uint8_t *)d_chars, ld, n, L, d_cols, nr, d_rep);
-    if ((e = cudaGetLastError()) != cudaSuccess) break;
-    for (int k = 0; k < nr; ++k) ptrs[k] = d_rep + (size_t)k * rep_bytes;
-    rc = rnj_batch_add_many(b, nr, ptrs.data(), ns.data(), Ls.data(), lds.data(), types.data(),
-                            models.data(), flags, d_out + r0, ldo.data(),
-                            slots.data());
+    if (!gathered) {
+      const long long work = (long long)nr * n * ((L + 3) / 4);
+      long long g = std::min<long long>((work + 255) / 256, 148LL * 32);
+      gather_columns_kernel<<<(unsigned)std::max<long long>(g, 1), 256, 0, ctx->stream>>>(
+          (const uint8_t *)d_chars, ld, n, L, d_cols, nr, d_rep);
+      if ((e = cudaGetLastError()) != cudaSuccess) break;
+    }
+    for (int k = 0; k < nr; ++k) ptrs[k] = gathered ? d_chars : d_rep + (size_t)k * rep_bytes;
+    rc = batch_add_many(b, nr, ptrs.data(), ns.data(), Ls.data(), lds.data(), types.data(),
+                        models.data(), flags, d_out + r0, ldo.data(), slots.data(),
+                        gathered ? d_cols : nullptr);
     if (rc == RNJ_OK) rc = rnj_batch_run(b);
     if (rc == RNJ_OK) rc = rnj_batch_synchronize(b);
     for (int k = 0; k < nr && rc == RNJ_OK; ++k)

@@ -194,6 +194,13 @@ cudaError_t launch_presence_multi(const PackJob *d_jobs, int njobs, long long un
                                   uint32_t *d_masks, cudaStream_t s);
 cudaError_t launch_pack_chars_multi(const PackJob *d_jobs, int njobs, long long units,
                                     cudaStream_t s);
+// `count` alignments whose site k is column d_cols[r * L + k] of d_chars, the features
+// of alignment r at F + r * stride (DNA; columns in range; L at most kMaxGatherColumns,
+// whose sites of eight rows still leave an SM two blocks).
+constexpr int kMaxGatherColumns = 24576;
+cudaError_t launch_pack_gathered(const uint8_t *d_chars, size_t ld, int n, int L, int Np, int Lk,
+                                 const int *d_cols, int count, size_t stride, uint8_t *F,
+                                 cudaStream_t s);
 cudaError_t launch_pack_features_multi(const PackJob *d_jobs, int njobs, long long units,
                                        cudaStream_t s);
 cudaError_t launch_pack_bitstrings_dna(const uint32_t *d_bits, const uint32_t *d_gaps,

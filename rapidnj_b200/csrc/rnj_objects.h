@@ -139,6 +139,13 @@ int distance_host_streamed(rnj_ctx *ctx, const char *chars, int n, int L, size_t
 // end 0 = begin), read back by rnj_ctx_stage_times.
 void ctx_mark(rnj_ctx *ctx, int stage, int end);
 
+// rnj_batch_add_many with the alignments' columns gathered from one (rnj_batch.cu):
+// site k of alignment r is column d_cols[r * L + k] of d_chars[0], which all entries
+// of d_chars name; DNA on the tensor-core layout, at most kMaxGatherColumns columns.
+int batch_add_many(rnj_batch *b, int count, const void *const *d_chars, const int *n, const int *L,
+                   const size_t *ld, const int *type, const int *model, int flags,
+                   float *const *d_out, const size_t *ld_out, int *slots, const int *d_cols);
+
 // A batch whose runs do not make the context stream wait (the server follows
 // completion through the batch's event and keeps packing the next batch).
 void batch_set_join(rnj_batch *b, bool join);

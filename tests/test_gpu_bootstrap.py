@@ -90,3 +90,23 @@ def test_rejects_bad_columns(ctx):
     d = torch.from_numpy(seqs).cuda()
     with pytest.raises(RnjError):
         ctx.bootstrap(d, np.full((2, 100), 100), 0, "kim")
+
+
+@pytest.mark.parametrize("n,L,R,pad", [(1, 1, 1, 0), (7, 8, 3, 3), (8, 255, 17, 0), (9, 256, 130, 1),
+                                       (129, 257, 33, 0), (130, 1000, 16, 5), (16, 24576, 3, 0),
+                                       (16, 24577, 3, 0)])
+def test_gathered_pack_at_its_edges(ctx, n, L, R, pad):
+    """The pack that gathers its columns: ragged rows and columns, any byte, strided
+    originals, replicates that do not fill a block, and the widest alignment it takes
+    and one wider.  Matrices equal the plain call's on the resampled bytes."""
+    rng = np.random.default_rng(n * L + R)
+    seqs = rng.choice(np.frombuffer(b"ACGTacgtU-N\xff", np.uint8), (n, L))
+    cols = rng.integers(0, L, (R, L)).astype(np.int32)
+    cols[0, 0], cols[-1, -1] = L - 1, 0
+    buf = torch.full((n, L + pad), ord("A"), dtype=torch.uint8, device="cuda")
+    buf[:, :L] = torch.from_numpy(seqs)
+    outs, mx = ctx.bootstrap(buf[:, :L], cols, 0, "kim")
+    for r in sorted({0, R // 2, R - 1}):
+        want, wmx = plain(ctx, np.ascontiguousarray(seqs[:, cols[r]]), 0, "kim")
+        assert np.array_equal(outs[r].cpu().numpy().view(np.int32), want.view(np.int32)), r
+        assert mx[r] == np.float32(wmx)
