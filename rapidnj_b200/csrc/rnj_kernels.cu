@@ -798,19 +798,37 @@ __global__ void __launch_bounds__(256) fixup_batch_kernel(const AlnDesc *__restr
                                                           const int *__restrict__ n_a,
                                                           const WorkItem *__restrict__ items_b,
                                                           const int *__restrict__ n_b) {
-  const int na = *n_a, nb = *n_b;
-  for (int it = blockIdx.x; it < na + nb; it += gridDim.x) {
-    const WorkItem w = it < na ? items_a[it] : items_b[it - na];
-    const AlnDesc &d = descs[w.aln];
-    if (d.out == nullptr) continue;
-    const float m2 = __fmul_rn(__int_as_float(*d.max_bits), 2.0f);
-    const int tile = w.tile & ~kPairSingle;
-    if (d.tile_flags[tile] != 0) fixup_tile<4>(d, tile, m2, threadIdx.x, blockDim.x);
-    if (!is_tc_kind(d.kind) || (w.tile & kPairSingle)) continue;
-    int ti, tj;
-    tri_coords(tile, d.nt, ti, tj);  // a row pair: the second row's tile
-    const int second = tile + d.nt - ti - 1;
-    if (ti < tj && d.tile_flags[second] != 0) fixup_tile<4>(d, second, m2, threadIdx.x, blockDim.x);
+  const int na = *n_a, nb = *n_b, lane = threadIdx.x & 31;
+  // The CTA's items are gridDim.x apart; every warp looks at 32 of them at a time, a
+  // lane each, so that the few flagged tiles are found in one round of loads.
+  for (long long base = blockIdx.x; base < na + nb; base += 32LL * gridDim.x) {
+    const long long at = base + (long long)lane * gridDim.x;
+    int aln = 0, first = -1, second = -1;  // flagged tiles of this lane's item
+    if (at < na + nb) {
+      const WorkItem w = at < na ? items_a[at] : items_b[at - na];
+      const AlnDesc &d = descs[w.aln];
+      aln = w.aln;
+      const int tile = w.tile & ~kPairSingle;
+      if (d.out != nullptr) {
+        if (d.tile_flags[tile] != 0) first = tile;
+        if (is_tc_kind(d.kind) && !(w.tile & kPairSingle)) {
+          int ti, tj;
+          tri_coords(tile, d.nt, ti, tj);  // a row pair: the second row's tile
+          const int next = tile + d.nt - ti - 1;
+          if (ti < tj && d.tile_flags[next] != 0) second = next;
+        }
+      }
+    }
+    uint32_t flagged = __ballot_sync(0xffffffffu, first >= 0 || second >= 0);
+    for (; flagged; flagged &= flagged - 1) {
+      const int src = __ffs(flagged) - 1;
+      const AlnDesc &d = descs[__shfl_sync(0xffffffffu, aln, src)];
+      const int t1 = __shfl_sync(0xffffffffu, first, src);
+      const int t2 = __shfl_sync(0xffffffffu, second, src);
+      const float m2 = __fmul_rn(__int_as_float(*d.max_bits), 2.0f);
+      if (t1 >= 0) fixup_tile<4>(d, t1, m2, threadIdx.x, blockDim.x);
+      if (t2 >= 0) fixup_tile<4>(d, t2, m2, threadIdx.x, blockDim.x);
+    }
   }
 }
 
