@@ -858,21 +858,20 @@ __device__ __forceinline__ void pair_produce(const TcShared &sh, int rank, const
 // The leader's MMA issuer (a whole warp): the same items as the producers.  Ends
 // after every MMA it issued has completed.
 //
-// Per stage there is only what must be: the MMAs and the commit, the next
-// stage's descriptor and a look at its barrier.
+// Per stage there is only what must be: a look at its barrier, the MMAs and the
+// commit, the next stage's descriptor.
 struct PairIssuer {
   const TcShared &sh;
   uint64_t desc0, desc;  // stage descriptors: the ring's first, the next K block's
   uint32_t tmem;
   int s;                 // stage of the next K block and the parity of its fill
   uint32_t ph;
-  bool ready, good;
+  bool good;
   uint64_t limit;
 
   __device__ __forceinline__ PairIssuer(const TcShared &sh_, uint32_t tmem_, uint64_t limit_)
       : sh(sh_), tmem(tmem_), s(0), ph(0), good(true), limit(limit_) {
     desc0 = desc = smem_desc_sw128(smem_u32(sh.stages));
-    ready = mbar_try_wait(&sh.full_bar[0], 0);
   }
   // Part k of the accumulators (0: V, 1: the rest) of the previous item has been
   // read in both CTAs.
@@ -891,7 +890,10 @@ struct PairIssuer {
     const uint32_t dt = tmem + (uint32_t)(acc * kTile);
     const uint32_t sfa = tmem + kTmemSfa, sfb = tmem + kTmemSfb;
     for (int kb = 0; kb < seg; kb += kPairBlocks) {
-      if (!__all_sync(0xffffffffu, ready)) {
+      // (Not before this stage is due: a try_wait holds its thread for microseconds
+      // while the phase is open, and one for the next stage, after an item's last,
+      // held back the commit of its accumulators by 4 us in every launch.)
+      if (!__all_sync(0xffffffffu, mbar_try_wait(&sh.full_bar[s], ph))) {
         int ok = 1;
         if ((threadIdx.x & 31) == 0) ok = tc_wait(&sh.full_bar[s], ph, sh.abort_flag, limit);
         good = __shfl_sync(0xffffffffu, ok, 0) != 0;
@@ -917,7 +919,6 @@ struct PairIssuer {
         ph ^= 1u;
         desc = desc0;
       }
-      ready = mbar_try_wait(&sh.full_bar[s], ph);
     }
   }
 };
