@@ -504,10 +504,10 @@ int run_tc_single(rnj_ctx *ctx, const Packed &p, const EpiParams &ep, int epi_mo
   const TuneParams tp = tune_lookup(p.n, p.L, p.type, p.flags);
   AlnDesc d = desc_for(p, ep);
   d.band = tp.tile_band;
-  if (epi_mode == EPI_COUNTS || !tc_fused_form(p, tp)) {
-    const int rc = encode_block_map(p, &d.map);
-    if (rc != RNJ_OK) return rc;
-  }
+  if (epi_mode != EPI_COUNTS && tc_fused_form(p, tp))
+    return run_tc_distances(ctx, p, ep, nullptr, ctx->stream, tp, &d);
+  const int rc = encode_block_map(p, &d.map);
+  if (rc != RNJ_OK) return rc;
   // Pageable source: the copy is taken before the call returns, so the stack
   // descriptor may go out of scope.
   RNJ_CUDA(cudaMemcpyAsync(ctx->d_desc, &d, sizeof(d), cudaMemcpyHostToDevice, ctx->stream),
@@ -565,7 +565,7 @@ int run_distance(rnj_ctx *ctx, const Packed &p, int model, float *d_out, size_t 
     mark(ctx, 1, 1);
     mark(ctx, 2, 0);
   }
-  RNJ_CUDA(launch_fixup(ep, nt, ctx->stream), "fix-up kernel");
+  RNJ_CUDA(launch_fixup(ep, nt, ctx->stream, is_tc_kind(p.kind)), "fix-up kernel");
   mark(ctx, 2, 1);
   if (d_max_copy)
     RNJ_CUDA(cudaMemcpyAsync(d_max_copy, ctx->scratch.words, sizeof(int), cudaMemcpyDeviceToDevice,
@@ -635,14 +635,14 @@ int ensure_packed(rnj_ctx *ctx, long long tiles) {
 }
 
 int run_tc_distances(rnj_ctx *ctx, const Packed &p, const EpiParams &ep, const AlnDesc *d_desc,
-                     cudaStream_t s, const TuneParams &tp) {
+                     cudaStream_t s, const TuneParams &tp, const AlnDesc *one) {
   if (tc_fused_form(p, tp)) {
     // Counts and transform in one launch (rnj_tcf.cu).
     mark(ctx, 1, 0);
     const int count = (int)pair_items(tiles_of(p.n));
     RNJ_CUDA(launch_tc_fused(d_desc, nullptr, 0, count,
                              fused_variant_for(ep.model, ep.type, ep.compat_wrap, 0), s,
-                             tp.tc_stages),
+                             tp.tc_stages, one),
              "fused tensor-core kernel");
     mark(ctx, 1, 1);
     mark(ctx, 2, 0);

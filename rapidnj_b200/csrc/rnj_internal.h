@@ -210,7 +210,9 @@ cudaError_t launch_pack_bitstrings_dna(const uint32_t *d_bits, const uint32_t *d
 cudaError_t launch_count_tiles(const Packed &p, int count_kind, int epi_mode,
                                const EpiParams &ep, cudaStream_t s, int kchunk = 0,
                                long long ntiles = 0);
-cudaError_t launch_fixup(const EpiParams &ep, int nt, cudaStream_t s);
+// after_fused: directly after the fused kernel on the stream, whose end it waits for
+// itself (its launch overlaps the kernel).
+cudaError_t launch_fixup(const EpiParams &ep, int nt, cudaStream_t s, bool after_fused = false);
 // Loads every bit-plane kernel a fused distance call can launch (pack, presence
 // scan, counts of each plane layout, fix-up).  Under CUDA's lazy module loading a
 // kernel's code is loaded, into device memory, at its first launch or attribute
@@ -264,13 +266,15 @@ cudaError_t launch_tc_transform(const AlnDesc *d_descs, const WorkItem *d_items,
 // flags.  Every alignment has at most kMaxFusedColumns columns.
 // variant: the transform of every item (fused_variant_for), or FUSED_ANY to
 // choose per item from its descriptor.  stages: the ring depth (0: the default, 6;
-// the tuner's tc_stages).
+// the tuner's tc_stages).  d_descs null: the one descriptor is `one` (host), which
+// goes along with the launch.
 enum FusedVariant {
   FUSED_K2P = 0, FUSED_JC = 1, FUSED_PROTEIN = 2, FUSED_GENERIC = 3, FUSED_FULL = 4, FUSED_ANY = 5
 };
 int fused_variant_for(int model, int type, int compat, int full);
 cudaError_t launch_tc_fused(const AlnDesc *d_descs, const WorkItem *d_items, int first, int count,
-                            int variant, cudaStream_t s, int stages = 0);
+                            int variant, cudaStream_t s, int stages = 0,
+                            const AlnDesc *one = nullptr);
 // Row-pair work items for launch_tc_fused: of the columns tj >= r0 of tile rows
 // [r0, r1), and of the tiles [t0, t1) in row-major order of the triangle.
 long long pair_items(int nt);  // items of a whole triangle of nt tile rows

@@ -578,6 +578,7 @@ __global__ void __launch_bounds__(256) transform_counts_kernel(int nt, EpiParams
 __global__ void __launch_bounds__(256, 8) fixup_kernel(int nt, EpiParams ep, int slices,
                                                        long long units) {
   const int lane = threadIdx.x & 31;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early: the fused kernel's end
   for (long long base = blockIdx.x; base < units; base += 32LL * gridDim.x) {
     const long long at = base + (long long)lane * gridDim.x;
     uint32_t flagged =
@@ -977,13 +978,21 @@ cudaError_t launch_count_tiles(const Packed &p, int count_kind, int epi_mode, co
   }
 }
 
-cudaError_t launch_fixup(const EpiParams &ep, int nt, cudaStream_t s) {
+cudaError_t launch_fixup(const EpiParams &ep, int nt, cudaStream_t s, bool after_fused) {
   const long long ntiles = ep.full ? (long long)nt * nt : tri_tiles(nt);
   if (ntiles == 0) return cudaSuccess;
   const int slices = ntiles <= 148 ? 16 : (ntiles <= 592 ? 4 : 1);
   const long long units = ntiles * slices;
-  fixup_kernel<<<(unsigned)std::min(units, 8 * 148LL), 256, 0, s>>>(nt, ep, slices, units);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3((unsigned)std::min(units, 8 * 148LL));
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = after_fused ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, fixup_kernel, nt, ep, slices, units);
 }
 
 cudaError_t launch_transform_counts(const EpiParams &ep, int nt, cudaStream_t s) {

@@ -78,9 +78,11 @@ inline bool tc_fused_form(const rnj::Packed &p, const rnj::TuneParams &tp) {
   return tp.tc_epilogue == 0 && p.L <= rnj::kMaxFusedColumns;
 }
 // Distances of the whole triangle of one tensor-core alignment (descriptor d_desc
-// on the device) by either form (rnj_api.cu).
+// on the device, or, for the fused form, null and `one` on the host) by either form
+// (rnj_api.cu).
 int run_tc_distances(rnj_ctx *ctx, const rnj::Packed &p, const rnj::EpiParams &ep,
-                     const rnj::AlnDesc *d_desc, cudaStream_t s, const rnj::TuneParams &tp);
+                     const rnj::AlnDesc *d_desc, cudaStream_t s, const rnj::TuneParams &tp,
+                     const rnj::AlnDesc *one = nullptr);
 
 struct rnj_aln {
   rnj_ctx *ctx = nullptr;

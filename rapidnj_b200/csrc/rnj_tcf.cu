@@ -96,13 +96,14 @@ struct TcfTables {
   float *stage;
 };
 
-// The tables into shared memory (every thread of the block; published by
-// tc_setup's block barriers).
+// The tables into shared memory, by the block's first kThreads threads (a barrier
+// of the caller publishes them).
+template <int kThreads>
 __device__ __forceinline__ TcfTables tcf_tables(const TcShared &sh) {
   uint8_t *const x = tc_extra(sh);
   double2 *const ln = reinterpret_cast<double2 *>(x);
   float *const pam = reinterpret_cast<float *>(x + kTcfTableBytes);
-  for (int e = threadIdx.x; e < kLnIntervals * kLnCopies; e += kTcfThreads)
+  for (int e = threadIdx.x; e < kLnIntervals * kLnCopies; e += kThreads)
     ln[e] = make_double2(__ldg(&c_log_tab_q[e / kLnCopies][0]), __ldg(&c_log_tab_q[e / kLnCopies][1]));
   if (threadIdx.x < 181) pam[threadIdx.x] = __ldg(c_pam.dist + threadIdx.x);
   return {ln + threadIdx.x % kLnCopies, pam,
@@ -574,12 +575,30 @@ __device__ __forceinline__ bool fused_tile(const TcShared &sh, uint32_t tmem, co
 
 // V: the transform variant of every item (kFused*), or kFusedAny to choose per
 // item (a work list of alignments with different models).  Items [first, last),
-// one per pair of CTAs at a time.
-template <int V>
+// one per pair of CTAs at a time.  kOne: one alignment, whose descriptor comes as a
+// parameter (its upload was a copy of its own before the launch) and whose items are
+// numbers; else the descriptors are in `list`.  (One kernel for both, with a pointer
+// to either, lost 1.5 % on large matrices: the fields were read again and again.)
+//
+// A call on a few hundred sequences is bound by what comes before the first load
+// and after the last MMA, so the producer waits for the barriers alone: tensor
+// memory's scale factors and the epilogue's tables are written while its first
+// loads are under way.  512 x 2,000 sites, JC: 35.6 -> 30.7 us for pack and distances
+// (copy, set-up and the early launch of the fix-up together); 50,000 x 1,000, K2P:
+// 5,500 -> 5,250, for the descriptor no longer takes registers.
+template <int V, bool kOne>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcfThreads, 1)
-    tc_fused_kernel(const AlnDesc *__restrict__ descs, const WorkItem *__restrict__ items,
-                    int first, int nitems, int nst) {
+    tc_fused_kernel(const AlnDesc *__restrict__ list, const WorkItem *__restrict__ list_items,
+                    int first, int nitems, int nst, const __grid_constant__ AlnDesc one) {
   extern __shared__ uint8_t smem_raw[];
+  const AlnDesc *const descs = kOne ? &one : list;
+  const WorkItem *const items = kOne ? nullptr : list_items;
+  // The fix-up that follows may be launched now; it waits for this grid's end.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (kOne && threadIdx.x == 0) {
+    prefetch_tmap(&one.map_a);
+    prefetch_tmap(&one.map_b);
+  }
   const TcShared sh = tc_shared(smem_raw, nst, kTcfExtra);
   const uint64_t limit = wait_limit_ns((uint32_t)descs[0].wait_us);
   const int stall = descs[0].stall;
@@ -589,7 +608,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcfThreads, 1)
   const int it0 = first + (int)(blockIdx.x >> 1), step = (int)(gridDim.x >> 1);
   if (it0 >= nitems) return;  // no item for this pair (both CTAs, before any setup)
 
-  const TcfTables tab = tcf_tables(sh);
   const uint32_t tmem = pair_setup(sh, kTcfEpiWarps, kTcfMmaWarp);
 
   if (warp >= kTcfProducerWarp) {
@@ -597,13 +615,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcfThreads, 1)
     // compiler allocates each role's code within its own limit.
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kTcfRegsLow) : "memory");
     if (warp == kTcfProducerWarp) {
-      if (lane == 0) pair_produce(sh, rank, descs, items, it0, nitems, step, limit);
-    } else if (warp == kTcfMmaWarp && rank == 0) {
-      pair_issue(sh, tmem, descs, items, it0, nitems, step, limit);
+      if (lane == 0) pair_produce(sh, rank, descs, items, it0, nitems, step, !kOne, limit);
+      __syncwarp();
+      cluster_wait();
+    } else {
+      cluster_wait();
+      tc_fence_after();
+      if (warp == kTcfMmaWarp && rank == 0)
+        pair_issue(sh, tmem, descs, items, it0, nitems, step, limit);
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kTcfRegsHigh) : "memory");
     // ----------------------------------------------------------- epilogue
+    const TcfTables tab = tcf_tables<32 * kTcfEpiWarps>(sh);
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kTcfEpiWarps) : "memory");  // its warps alone
+    cluster_wait();
+    tc_fence_after();
     uint32_t titer = 0;
     PairWalk walk(descs, items, rank);
     float seen = 0.0f;
@@ -776,7 +803,7 @@ __global__ void __launch_bounds__(kTcfThreads, 1)
   const uint64_t limit = wait_limit_ns((uint32_t)descs[0].wait_us);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  const TcfTables tab = tcf_tables(sh);
+  const TcfTables tab = tcf_tables<kTcfThreads>(sh);  // published by tc_setup's block barriers
   if (tid == 0) {
     for (int k = 0; k < 2; ++k) {
       mbar_init(&lr->full[k], 1);
@@ -1027,31 +1054,32 @@ static int max_pairs(int device, cudaError_t *err) {
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int n = 0;
-  *err = cudaOccupancyMaxActiveClusters(&n, tc_fused_kernel<kFusedK2p>, &cfg);
+  *err = cudaOccupancyMaxActiveClusters(&n, tc_fused_kernel<kFusedK2p, false>, &cfg);
   if (*err != cudaSuccess) return 0;
   n = std::max(1, n);
   if (keep) known[device].store(n, std::memory_order_relaxed);
   return n;
 }
 
-template <int V>
+template <int V, bool kOne>
 static cudaError_t launch_variant(const AlnDesc *d_descs, const WorkItem *d_items,
-                                  int first, int count, int stages, cudaStream_t s) {
+                                  int first, int count, int stages, cudaStream_t s,
+                                  const AlnDesc &one) {
   const int nst = pair_stages(stages);
   const size_t smem = tc_smem_bytes(nst, kTcfExtra, kPairStageBytes);
   int device = 0;
   cudaError_t e = cudaGetDevice(&device);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(tc_fused_kernel<kFusedK2p>,
+    e = cudaFuncSetAttribute(tc_fused_kernel<kFusedK2p, false>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcfSmemBytes);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(tc_fused_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(tc_fused_kernel<V, kOne>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kTcfSmemBytes);
   if (e != cudaSuccess) return e;
   const int pairs = std::min(count, max_pairs(device, &e));
   if (e != cudaSuccess) return e;
-  tc_fused_kernel<V><<<(unsigned)(2 * pairs), kTcfThreads, smem, s>>>(
-      d_descs, d_items, first, first + count, nst);
+  tc_fused_kernel<V, kOne><<<(unsigned)(2 * pairs), kTcfThreads, smem, s>>>(
+      d_descs, d_items, first, first + count, nst, one);
   return cudaGetLastError();
 }
 
@@ -1065,15 +1093,23 @@ int fused_variant_for(int model, int type, int compat, int full) {
 int fused_ring_depth(int stages) { return tc_ring_depth(stages, kTcfStages, kTcfStages); }
 
 cudaError_t launch_tc_fused(const AlnDesc *d_descs, const WorkItem *d_items, int first, int count,
-                            int variant, cudaStream_t s, int stages) {
+                            int variant, cudaStream_t s, int stages, const AlnDesc *one) {
   if (count <= 0) return cudaSuccess;
-  using Launch = cudaError_t (*)(const AlnDesc *, const WorkItem *, int, int, int, cudaStream_t);
-  // indexed by FusedVariant
-  static const Launch kLaunch[] = {launch_variant<kFusedK2p>, launch_variant<kFusedJc>,
-                                   launch_variant<kFusedProtein>, launch_variant<kFusedGeneric>,
-                                   launch_variant<kFusedFull>, launch_variant<kFusedAny>};
-  if (variant < FUSED_K2P || variant > FUSED_ANY) return cudaErrorInvalidValue;
-  return kLaunch[variant](d_descs, d_items, first, count, stages, s);
+  if (!d_descs == !one) return cudaErrorInvalidValue;
+  using Launch = cudaError_t (*)(const AlnDesc *, const WorkItem *, int, int, int, cudaStream_t,
+                                 const AlnDesc &);
+  // indexed by FusedVariant (one alignment's calls have its own variant)
+  static const Launch kList[] = {
+      launch_variant<kFusedK2p, false>,     launch_variant<kFusedJc, false>,
+      launch_variant<kFusedProtein, false>, launch_variant<kFusedGeneric, false>,
+      launch_variant<kFusedFull, false>,    launch_variant<kFusedAny, false>};
+  static const Launch kSingle[] = {
+      launch_variant<kFusedK2p, true>, launch_variant<kFusedJc, true>,
+      launch_variant<kFusedProtein, true>, launch_variant<kFusedGeneric, true>};
+  if (variant < FUSED_K2P || variant > (one ? FUSED_GENERIC : FUSED_ANY) || (one && d_items))
+    return cudaErrorInvalidValue;
+  if (one) return kSingle[variant](nullptr, nullptr, first, count, stages, s, *one);
+  return kList[variant](d_descs, d_items, first, count, stages, s, AlnDesc{});
 }
 
 long long pair_items(int nt) {

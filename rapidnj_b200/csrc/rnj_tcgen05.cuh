@@ -136,6 +136,14 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
                ::: "memory");
 }
+// Its two halves (whole warps): a warp that need not see the others' writes yet
+// arrives, and waits before its next arrival.
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // The cluster address of this shared-memory address in CTA `rank`.
 __device__ __forceinline__ uint32_t cluster_addr(const void *p, uint32_t rank) {
   uint32_t a;
@@ -771,9 +779,11 @@ __device__ __forceinline__ void pair_abort(const TcShared &sh) {
                  : "memory");
 }
 
-// As tc_setup, for both CTAs (ends with a cluster barrier: no CTA arrives on, or
-// loads towards, the other's barriers before they are set up).  warps: epilogue
-// warps of a CTA; warps 0 .. 7 fill the scale-factor columns.
+// As tc_setup, for both CTAs, with a cluster barrier (no CTA arrives on, or loads
+// towards, the other's barriers before they are set up).  warps: epilogue warps of a
+// CTA; warps 0 .. 7 fill the scale-factor columns.  Ends with the arrival on a second
+// cluster barrier: cluster_wait, then tc_fence_after, before tensor memory is used;
+// loads need not wait for that.
 __device__ __forceinline__ uint32_t pair_setup(const TcShared &sh, uint32_t warps, int alloc_warp) {
   const int tid = threadIdx.x, warp = tid >> 5;
   if (tid == 0) {
@@ -793,7 +803,7 @@ __device__ __forceinline__ uint32_t pair_setup(const TcShared &sh, uint32_t warp
   }
   if (warp == alloc_warp) tmem_alloc_pair(sh.tmem_slot, kTmemCols);
   tc_fence_before();
-  __syncthreads();
+  cluster_sync();
   tc_fence_after();
   const uint32_t tmem = *sh.tmem_slot;
   if (warp < 8) {
@@ -804,9 +814,7 @@ __device__ __forceinline__ uint32_t pair_setup(const TcShared &sh, uint32_t warp
     tmem_st_wait();
   }
   tc_fence_before();
-  __syncthreads();
-  cluster_sync();
-  tc_fence_after();
+  cluster_arrive();
   return tmem;
 }
 
@@ -824,9 +832,10 @@ __device__ __forceinline__ void pair_load(const TcShared &sh, int rank, uint32_t
 }
 
 // The producer (one thread of each CTA): items it0, it0 + step, ... below nitems.
+// acquire: the descriptors' tensor maps are in global memory, written by a copy.
 __device__ __forceinline__ void pair_produce(const TcShared &sh, int rank, const AlnDesc *descs,
                                              const WorkItem *items, int it0, int nitems, int step,
-                                             uint64_t limit) {
+                                             bool acquire, uint64_t limit) {
   const uint32_t bar0 = cluster_addr(sh.full_bar, 0);
   uint32_t issued = 0, pph = 0;  // stages loaded, parity of the next fill
   int s = 0;                     // its stage
@@ -835,8 +844,10 @@ __device__ __forceinline__ void pair_produce(const TcShared &sh, int rank, const
   for (int it = it0; good && it < nitems && !*sh.abort_flag; it += step) {
     const TileAt t = walk.at(it);
     const AlnDesc &d = descs[t.aln];
-    tensormap_acquire(&d.map_a);
-    tensormap_acquire(&d.map_b);
+    if (acquire) {
+      tensormap_acquire(&d.map_a);
+      tensormap_acquire(&d.map_b);
+    }
     const int seg = d.kdim / kTcKCols, np = d.np;
     const int row_a = t.ti * kTile, row_b = t.tj * kTile + rank * (kTile / 2);
     for (int f = 0; good && f < np; ++f) {
