@@ -333,11 +333,11 @@ __device__ __forceinline__ float valid_of(uint32_t pv, int k) {
   return __fsub_rn(valid23_of(pv, k), 8388608.0f);
 }
 
-// Sixteen columns of row i, from jb: pv the valid counts (two a word), ar and at
+// Sixteen columns (kGroups 1: eight) of row i, from jb: pv the valid counts (two a word), ar and at
 // the other accumulators' words.  Eight at a time: a group of the warp's rows and
 // eight columns lies above the diagonal and inside the matrix (no masks), or
 // holds nothing of the triangle (skipped), or straddles an edge.
-template <int M, bool kProt>
+template <int M, bool kProt, int kGroups>
 __device__ __forceinline__ void fused_cols(const AlnDesc &d, float *out, size_t ld, int n, int i,
                                            int jb, RowStore how, const uint32_t (&pv)[16], const uint32_t (&ar)[16],
                                            const uint32_t (&at)[16], float &tmax, float &tmin,
@@ -345,7 +345,7 @@ __device__ __forceinline__ void fused_cols(const AlnDesc &d, float *out, size_t 
                                            const TcfTables &tab) {
   const int ilo = i - (int)(threadIdx.x & 31);  // the warp's first row
 #pragma unroll
-  for (int g = 0; g < 2; ++g) {
+  for (int g = 0; g < kGroups; ++g) {
     const int j0 = jb + 8 * g;
     if (j0 + 7 < ilo || j0 >= n || ilo >= n) continue;
     const bool interior = ilo + 31 < j0 && j0 + 7 < n && (ld >> 32) == 0;
@@ -462,23 +462,26 @@ __device__ __forceinline__ bool skip_tile(const TcShared &sh, uint32_t titer, in
   return true;
 }
 
-// One tile of the epilogue (every epilogue warp; warp w reads tensor-memory
-// lane quarter w % 4 and columns 32 (w / 4) .. + 31): waits for V of the CTA's
+// One tile of the epilogue, or slice `slice` of 32 / kCols of its columns (every
+// epilogue warp; warp w reads tensor-memory lane quarter w % 4 and columns kCols
+// (w / 4) .. + kCols - 1): waits for V of the CTA's
 // item number titer and hands it back, then for the other accumulators, which
 // go back once their second half is in registers; the transform, the stores,
 // the tile's maximum (through the alignment's max slot when it exceeds `seen`,
 // the largest this warp has sent there) and saturation flag.  False when a wait
 // ran out (the caller sets the abort flag).
-template <int M, bool kProt, bool kPair>
+template <int M, bool kProt, bool kPair, int kCols>
 __device__ __forceinline__ bool fused_tile_as(const TcShared &sh, uint32_t tmem, const AlnDesc &d,
                                            const TileAt &t, uint32_t titer, int stall,
                                            uint64_t limit, const TcfTables &tab, float &seen,
-                                           int *sat_any = nullptr) {
+                                           int slice, int *sat_any = nullptr) {
+  constexpr int kRounds = kCols > 16 ? kCols / 16 : 1;
+  static_assert(kCols == 32 || kCols == 16 || kCols == 8, "columns of a warp");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q = warp & 3;              // tensor-memory lane quarter
-  const int cofs = 32 * (warp >> 2);   // first tile column of this warp
+  const int q = warp & 3;                // tensor-memory lane quarter
+  const int cofs = kCols * (warp >> 2);  // this warp's first column of the accumulators
   const int i = t.ti * kTile + 32 * q + lane;  // this lane's row
-  const int jb = t.tj * kTile + cofs;
+  const int jb = t.tj * kTile + 4 * kCols * slice + cofs;
   const uint32_t base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)cofs;
   // The descriptor's fields, read once (every store below could have changed
   // them, for all the compiler knows).
@@ -499,12 +502,13 @@ __device__ __forceinline__ bool fused_tile_as(const TcShared &sh, uint32_t tmem,
   // of which go into a word.
   uint32_t pv[16];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < kRounds; ++h) {
     uint32_t av[16];
-    tmem_ld16(base + 16 * h, av);
+    if constexpr (kCols == 8) tmem_ld8(base, av);
+    else tmem_ld16(base + 16 * h, av);
     tmem_ld_wait();
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
+    for (int k = 0; k < (kCols == 8 ? 4 : 8); ++k)
       pv[8 * h + k] = __byte_perm(
           __float_as_uint(__fadd_rn(__uint_as_float(av[2 * k]), 8388608.0f)),
           __float_as_uint(__fadd_rn(__uint_as_float(av[2 * k + 1]), 8388608.0f)), 0x5410);
@@ -517,23 +521,30 @@ __device__ __forceinline__ bool fused_tile_as(const TcShared &sh, uint32_t tmem,
 
   float tmax = 0.0f, tmin = 0.0f;
 #pragma unroll 1
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < kRounds; ++h) {
     uint32_t ar[16], at[16];
-    tmem_ld16(base + kTile + 16 * h, ar);
-    tmem_ld16(base + 2 * kTile + 16 * h, at);
+    if constexpr (kCols == 8) {
+      tmem_ld8(base + kTile, ar);
+      tmem_ld8(base + 2 * kTile, at);
+    } else {
+      tmem_ld16(base + kTile + 16 * h, ar);
+      tmem_ld16(base + 2 * kTile + 16 * h, at);
+    }
     tmem_ld_wait();
-    if (h == 1) {
+    if (h == kRounds - 1) {
       tc_fence_before();
       __syncwarp();
       if (lane == 0) arrive_read<kPair>(sh, 1);
+      if constexpr (kRounds == 2) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) pv[k] = pv[k + 8];
+        for (int k = 0; k < 8; ++k) pv[k] = pv[k + 8];
+      }
     }
     const int jh = jb + 16 * h;
     if constexpr (M == kFusedFull)
       fused_cols_full(d, i, jh, pv, ar, at, tmax, tmin);
     else
-      fused_cols<M, kProt>(d, out, ld, n, i, jh, how, pv, ar, at, tmax, tmin, inv_b, rc,
+      fused_cols<M, kProt, kCols == 8 ? 1 : 2>(d, out, ld, n, i, jh, how, pv, ar, at, tmax, tmin, inv_b, rc,
                            tab);
   }
   // (non-negative floats order as their bits)
@@ -552,13 +563,13 @@ __device__ __forceinline__ bool fused_tile_as(const TcShared &sh, uint32_t tmem,
 
 // The tile by its variant: each model's code on its own, so that none keeps
 // another's parameters in registers.
-template <int V, bool kPair>
+template <int V, bool kPair, int kCols = 32>
 __device__ __forceinline__ bool fused_tile(const TcShared &sh, uint32_t tmem, const AlnDesc &d,
                                            const TileAt &t, uint32_t titer, int stall,
                                            uint64_t limit, const TcfTables &tab, float &seen,
-                                           int *sat_any = nullptr) {
+                                           int slice, int *sat_any = nullptr) {
 #define RNJ_TILE(M, P) \
-  fused_tile_as<M, P, kPair>(sh, tmem, d, t, titer, stall, limit, tab, seen, sat_any)
+  fused_tile_as<M, P, kPair, kCols>(sh, tmem, d, t, titer, stall, limit, tab, seen, slice, sat_any)
   if constexpr (V == kFusedFull) return RNJ_TILE(kFusedFull, false);
   else if constexpr (V == kFusedK2p) return RNJ_TILE(kFusedK2p, false);
   else if constexpr (V == kFusedProtein) return RNJ_TILE(kFusedProtein, true);
@@ -586,7 +597,12 @@ __device__ __forceinline__ bool fused_tile(const TcShared &sh, uint32_t tmem, co
 // loads are under way.  512 x 2,000 sites, JC: 35.6 -> 30.7 us for pack and distances
 // (copy, set-up and the early launch of the fix-up together); 50,000 x 1,000, K2P:
 // 5,500 -> 5,250, for the descriptor no longer takes registers.
-template <int V, bool kOne>
+//
+// kSlices: a tile is that many items, each with 128 / kSlices of its columns.  Few
+// tiles leave most SMs idle, and a tile's epilogue (14k cycles) is then half of the
+// kernel; the rows' features are read once per slice instead.  512 x 2,000, pack and
+// distances: 30.7 -> 26.9 us; 301 x 421 residues: 52.5 -> 46.4.
+template <int V, bool kOne, int kSlices>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcfThreads, 1)
     tc_fused_kernel(const AlnDesc *__restrict__ list, const WorkItem *__restrict__ list_items,
                     int first, int nitems, int nst, const __grid_constant__ AlnDesc one) {
@@ -615,14 +631,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcfThreads, 1)
     // compiler allocates each role's code within its own limit.
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kTcfRegsLow) : "memory");
     if (warp == kTcfProducerWarp) {
-      if (lane == 0) pair_produce(sh, rank, descs, items, it0, nitems, step, !kOne, limit);
+      if (lane == 0)
+        pair_produce<kSlices>(sh, rank, descs, items, it0, nitems, step, !kOne, limit);
       __syncwarp();
       cluster_wait();
     } else {
       cluster_wait();
       tc_fence_after();
       if (warp == kTcfMmaWarp && rank == 0)
-        pair_issue(sh, tmem, descs, items, it0, nitems, step, limit);
+        pair_issue<kSlices>(sh, tmem, descs, items, it0, nitems, step, limit);
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kTcfRegsHigh) : "memory");
@@ -636,15 +653,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcfThreads, 1)
     float seen = 0.0f;
     int last = 0;
     for (int it = it0; it < nitems; it += step, ++titer) {
-      const TileAt t = walk.at(it);
+      const TileAt t = walk.at(it / kSlices);
       if (t.aln != last) {
         last = t.aln;
         seen = 0.0f;
       }
       const bool ok = t.tile < 0
                           ? skip_tile(sh, titer, stall, limit)
-                          : fused_tile<V, true>(sh, tmem, descs[t.aln], t, titer, stall, limit,
-                                                tab, seen);
+                          : fused_tile<V, true, 32 / kSlices>(sh, tmem, descs[t.aln], t, titer,
+                                                              stall, limit, tab, seen, it % kSlices);
       if (!ok) {
         pair_abort(sh);
         break;
@@ -935,7 +952,7 @@ __global__ void __launch_bounds__(kTcfThreads, 1)
       TileAt t{aln, tile, 0, 0};
       item_tile(d, tile, t.ti, t.tj);
       float seen = 0.0f;
-      if (!fused_tile<kFusedAny, false>(sh, tmem, d, t, titer, 0, limit, tab, seen,
+      if (!fused_tile<kFusedAny, false>(sh, tmem, d, t, titer, 0, limit, tab, seen, 0,
                                        &live.sat[aln])) {
         *sh.abort_flag = 1;
         break;
@@ -1054,14 +1071,14 @@ static int max_pairs(int device, cudaError_t *err) {
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int n = 0;
-  *err = cudaOccupancyMaxActiveClusters(&n, tc_fused_kernel<kFusedK2p, false>, &cfg);
+  *err = cudaOccupancyMaxActiveClusters(&n, tc_fused_kernel<kFusedK2p, false, 1>, &cfg);
   if (*err != cudaSuccess) return 0;
   n = std::max(1, n);
   if (keep) known[device].store(n, std::memory_order_relaxed);
   return n;
 }
 
-template <int V, bool kOne>
+template <int V, bool kOne, int kSlices>
 static cudaError_t launch_variant(const AlnDesc *d_descs, const WorkItem *d_items,
                                   int first, int count, int stages, cudaStream_t s,
                                   const AlnDesc &one) {
@@ -1070,15 +1087,23 @@ static cudaError_t launch_variant(const AlnDesc *d_descs, const WorkItem *d_item
   int device = 0;
   cudaError_t e = cudaGetDevice(&device);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(tc_fused_kernel<kFusedK2p, false>,
+    e = cudaFuncSetAttribute(tc_fused_kernel<kFusedK2p, false, 1>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcfSmemBytes);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(tc_fused_kernel<V, kOne>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(tc_fused_kernel<V, kOne, kSlices>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kTcfSmemBytes);
   if (e != cudaSuccess) return e;
-  const int pairs = std::min(count, max_pairs(device, &e));
+  const int most = max_pairs(device, &e);
   if (e != cudaSuccess) return e;
-  tc_fused_kernel<V, kOne><<<(unsigned)(2 * pairs), kTcfThreads, smem, s>>>(
+  if constexpr (kOne && kSlices < 4) {
+    // Slices while every one gets a pair of CTAs of its own.
+    if (count * 2 * kSlices <= most)
+      return launch_variant<V, kOne, 2 * kSlices>(d_descs, d_items, first, count, stages, s, one);
+  }
+  first *= kSlices;
+  count *= kSlices;
+  const int pairs = std::min(count, most);
+  tc_fused_kernel<V, kOne, kSlices><<<(unsigned)(2 * pairs), kTcfThreads, smem, s>>>(
       d_descs, d_items, first, first + count, nst, one);
   return cudaGetLastError();
 }
@@ -1100,12 +1125,12 @@ cudaError_t launch_tc_fused(const AlnDesc *d_descs, const WorkItem *d_items, int
                                  const AlnDesc &);
   // indexed by FusedVariant (one alignment's calls have its own variant)
   static const Launch kList[] = {
-      launch_variant<kFusedK2p, false>,     launch_variant<kFusedJc, false>,
-      launch_variant<kFusedProtein, false>, launch_variant<kFusedGeneric, false>,
-      launch_variant<kFusedFull, false>,    launch_variant<kFusedAny, false>};
+      launch_variant<kFusedK2p, false, 1>,     launch_variant<kFusedJc, false, 1>,
+      launch_variant<kFusedProtein, false, 1>, launch_variant<kFusedGeneric, false, 1>,
+      launch_variant<kFusedFull, false, 1>,    launch_variant<kFusedAny, false, 1>};
   static const Launch kSingle[] = {
-      launch_variant<kFusedK2p, true>, launch_variant<kFusedJc, true>,
-      launch_variant<kFusedProtein, true>, launch_variant<kFusedGeneric, true>};
+      launch_variant<kFusedK2p, true, 1>, launch_variant<kFusedJc, true, 1>,
+      launch_variant<kFusedProtein, true, 1>, launch_variant<kFusedGeneric, true, 1>};
   if (variant < FUSED_K2P || variant > (one ? FUSED_GENERIC : FUSED_ANY) || (one && d_items))
     return cudaErrorInvalidValue;
   if (one) return kSingle[variant](nullptr, nullptr, first, count, stages, s, *one);

@@ -227,8 +227,11 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
 // UE8M0 (bit 23), M >> 4 at bits 24-28, scale-factor ids 0, dense K = 64.
 constexpr uint32_t kIdescFp4 = (1u << 7) | (1u << 10) | ((uint32_t)(kTile >> 3) << 17) | (1u << 23) |
                                ((uint32_t)(kTile >> 4) << 24);
-constexpr uint32_t kIdescFp4Pair = (1u << 7) | (1u << 10) | ((uint32_t)(kTile >> 3) << 17) |
-                                   (1u << 23) | ((uint32_t)(2 * kTile >> 4) << 24);  // M = 256
+// M = 256, N = a tile's columns or a slice of them
+template <int kSlices>
+constexpr uint32_t kIdescFp4Pair = (1u << 7) | (1u << 10) |
+                                   ((uint32_t)(kTile / kSlices >> 3) << 17) | (1u << 23) |
+                                   ((uint32_t)(2 * kTile >> 4) << 24);
 
 // A bounded wait (limit_ns) that also gives up early once another role has
 // aborted.  Between tests the thread sleeps until the phase completes, for at
@@ -254,6 +257,14 @@ __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, volatile
 }
 
 // 32 lanes x 16 columns of 32-bit words from tensor memory into registers.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[16]) {  // eight columns
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
@@ -833,6 +844,9 @@ __device__ __forceinline__ void pair_load(const TcShared &sh, int rank, uint32_t
 
 // The producer (one thread of each CTA): items it0, it0 + step, ... below nitems.
 // acquire: the descriptors' tensor maps are in global memory, written by a copy.
+// kSlices: every tile is that many items, each with its share of the columns (the
+// box of B is loaded whole, the MMAs read the rows of the slice).
+template <int kSlices>
 __device__ __forceinline__ void pair_produce(const TcShared &sh, int rank, const AlnDesc *descs,
                                              const WorkItem *items, int it0, int nitems, int step,
                                              bool acquire, uint64_t limit) {
@@ -842,14 +856,15 @@ __device__ __forceinline__ void pair_produce(const TcShared &sh, int rank, const
   PairWalk walk(descs, items, rank);
   bool good = true;
   for (int it = it0; good && it < nitems && !*sh.abort_flag; it += step) {
-    const TileAt t = walk.at(it);
+    const TileAt t = walk.at(it / kSlices);
     const AlnDesc &d = descs[t.aln];
     if (acquire) {
       tensormap_acquire(&d.map_a);
       tensormap_acquire(&d.map_b);
     }
     const int seg = d.kdim / kTcKCols, np = d.np;
-    const int row_a = t.ti * kTile, row_b = t.tj * kTile + rank * (kTile / 2);
+    const int row_a = t.ti * kTile;
+    const int row_b = t.tj * kTile + (2 * (it % kSlices) + rank) * (kTile / 2 / kSlices);
     for (int f = 0; good && f < np; ++f) {
       for (int kb = 0; kb < seg; kb += kPairBlocks) {
         if (!(good = tc_wait(&sh.empty_bar[s], pph ^ 1u, sh.abort_flag, limit))) break;
@@ -871,6 +886,7 @@ __device__ __forceinline__ void pair_produce(const TcShared &sh, int rank, const
 //
 // Per stage there is only what must be: a look at its barrier, the MMAs and the
 // commit, the next stage's descriptor.
+template <int kSlices>
 struct PairIssuer {
   const TcShared &sh;
   uint64_t desc0, desc;  // stage descriptors: the ring's first, the next K block's
@@ -912,15 +928,15 @@ struct PairIssuer {
       }
       const uint64_t ad = desc, bd = desc + (kPairABytes >> 4);
       // 32 bytes = 64 columns per MMA, four per 128-byte K block.
-      tc_mma_fp4_pair_elect(dt, ad, bd, kIdescFp4Pair, sfa, sfb, accumulate);
+      tc_mma_fp4_pair_elect(dt, ad, bd, kIdescFp4Pair<kSlices>, sfa, sfb, accumulate);
 #pragma unroll
       for (int j = 1; j < 4; ++j)
-        tc_mma_fp4_pair_elect(dt, ad + 2 * j, bd + 2 * j, kIdescFp4Pair, sfa, sfb, 1u);
+        tc_mma_fp4_pair_elect(dt, ad + 2 * j, bd + 2 * j, kIdescFp4Pair<kSlices>, sfa, sfb, 1u);
       if (kb + 1 < seg) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          tc_mma_fp4_pair_elect(dt, ad + kAStep + 2 * j, bd + kBStep + 2 * j, kIdescFp4Pair, sfa,
-                                sfb, 1u);
+          tc_mma_fp4_pair_elect(dt, ad + kAStep + 2 * j, bd + kBStep + 2 * j,
+                                kIdescFp4Pair<kSlices>, sfa, sfb, 1u);
       }
       tc_commit_pair_elect(&sh.empty_bar[s]);
       accumulate = 1u;
@@ -934,11 +950,12 @@ struct PairIssuer {
   }
 };
 
+template <int kSlices>
 __device__ __forceinline__ void pair_issue(const TcShared &sh, uint32_t tmem, const AlnDesc *descs,
                                            const WorkItem *items, int it0, int nitems, int step,
                                            uint64_t limit) {
   const int lane = threadIdx.x & 31;
-  PairIssuer is(sh, tmem, limit);
+  PairIssuer<kSlices> is(sh, tmem, limit);
   uint32_t titer = 0;
   for (int it = it0; is.good; it += step, ++titer) {
     int go = it < nitems && !*sh.abort_flag;

@@ -82,3 +82,23 @@ def test_batch_of_every_variant(ctx):
     for w, slot in zip(want, slots):
         assert np.array_equal(b.take(slot).to_numpy().view(np.int32), w.view(np.int32))
     b.close()
+
+
+@pytest.mark.parametrize("typ,model,wrap", [(0, "kim", False), (0, "jc", False), (1, "kim", False),
+                                            (1, "jc", False), (1, "kim", True)])
+@pytest.mark.parametrize("n", [2, 129, 897, 1025, 1409, 1700])
+def test_column_slices(ctx, typ, model, wrap, n):
+    """Plain calls around the sizes at which their tiles are split into column slices
+    against the batch's whole tiles: bit for bit, the maximum too."""
+    from rapidnj_b200 import api
+    s = alignment(typ, n, 640, seed=n + typ)
+    a = ctx.alignment(s, typ, compat_wrap=wrap)
+    out = torch.full((n, n + 3), -7.0, dtype=torch.float32, device="cuda")
+    mx = ctx.distance_into(a, model, out, want_max=True)
+    with_batch = api.Batch(ctx, max_alignments=1, max_tiles=4096)
+    slot = with_batch.add(a, model)
+    with_batch.run()
+    want = with_batch.take(slot).to_numpy()
+    assert np.array_equal(out[:, :n].cpu().numpy().view(np.int32), want.view(np.int32))
+    assert np.float32(mx) == np.float32(with_batch.max(slot))
+    assert bool((out[:, n:] == -7.0).all())
