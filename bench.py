@@ -382,7 +382,7 @@ def run_batched(args, local_rank: int = 0, count: int = 256):
     """The mixed workload (N ~ U[32, 2048], L ~ U[300, 5000], 70 % tree DNA
     Kimura-2P, 30 % tree protein Kimura): plain per-request calls (pack +
     rnj_distance_into per alignment) against one batched pass (pack each, one
-    graph-captured persistent launch over all tiles).  Inputs resident; outputs
+    persistent launch over all tiles).  Inputs resident; outputs
     preallocated; the matrices of both must be identical."""
     import torch
     from rapidnj_b200 import api, synth
