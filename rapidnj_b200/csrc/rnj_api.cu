@@ -311,7 +311,7 @@ void lut_for(int type, int flags, const uint32_t *mask, uint8_t lut[256], int *k
 }
 
 // The scan reports straight to page-locked memory and leaves its words clear: one
-// launch and a wait, 61 us for pack and distances of 301 x 421 residues against 70 with a
+// launch and a wait; pack and distances of 301 x 421 residues took 61 us with it and 70 with a
 // clear, the scan and a copy.
 int presence_mask(rnj_ctx *ctx, const uint8_t *d_chars, int n, int L, size_t ld) {
   memset(ctx->h_mask, 0, 8 * sizeof(uint32_t));
@@ -331,8 +331,8 @@ namespace {
 // fast rules' kernels.  The two rules count alike unless lower-case a/c/g/t or U in
 // either case occur (valid sites whose differences the naive rule classifies by the
 // row's case).  The plane kernel, with a population count per word and pair, then
-// gives way to the tensor cores: 3,001 x 4,003 sites 873 -> 115 us, 500 x 2,000 191 ->
-// 59, 3,000 x 60 214 -> 85.  Letters that need the planes cost the call the scan and
+// gives way to the tensor cores: 3,001 x 4,003 sites 880 -> 105 us, 500 x 2,000 191 ->
+// 45, 3,000 x 60 214 -> 82.  Letters that need the planes cost the call the scan and
 // its wait, 16 us, so the scan is kept to where the planes take 150 us or more: many
 // columns (60 us + 0.06 a column, whatever the rows) or many rows.  Under stream
 // capture there is no waiting for the scan; whole rows (FULL_ROWS) and calls that ask

@@ -35,11 +35,12 @@
 //
 // What bounds it.  Long alignments: the MMAs of a pair, 326 cycles per 256
 // columns with operands at rest, 343 with loads, 436 with the epilogue at work
-// (10,000 x 10,000 DNA step 1.00 -> 0.955 ms; the chip is at its 1,000 W limit
-// there, 1.76 GHz).  Short ones: the epilogue, 18,000 cycles a tile for the K2P
-// transform, 73 warp instructions per 32 pairs (168 before: 50,000 x 1,000 step
-// 7.58 -> 5.79 ms), no pipe above a third of its rate; of what it does, the
-// stores cost 15 %, the table reads 9 %, each double operation about 1.7 %.
+// (10,000 x 10,000 DNA call 1.007 -> 0.912 ms; the chip is at its 1,000 W limit
+// there, 1.76 GHz).  Short ones: the epilogue, 69 warp instructions per 32 K2P
+// pairs (168 before: 50,000 x 1,000 call 7.55 -> 5.28 ms) at 0.46 issues a cycle
+// with four warps a scheduler, no pipe above a quarter of its rate; of what it
+// does, the stores cost 15 %, the table reads 9 %, each double operation about
+// 1.7 %.  Few tiles: set-up and one tile's latency (kSlices, tc_fused_kernel).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
