@@ -314,7 +314,8 @@ int rnj_batch_synchronize(rnj_batch *batch);
 /* Non-blocking: *done = 1 once the last run has completed on the device. */
 int rnj_batch_poll(rnj_batch *batch, int *done);
 /* The output of a slot (device pointer and stride); max_out (may be NULL)
- * waits for the run and reads the slot's maximum distance. */
+ * waits for the run and reads the slot's maximum distance (0 for a slot that the
+ * last run did not hold: added after it, or none has run). */
 int rnj_batch_output(rnj_batch *batch, int slot, float **d_out, size_t *ld, float *max_out);
 /* Moves a batch-allocated output into a matrix handle (for rnj_mat_copy_rows). */
 int rnj_batch_take(rnj_batch *batch, int slot, rnj_mat **out);

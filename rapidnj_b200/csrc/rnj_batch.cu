@@ -60,6 +60,7 @@ struct rnj_batch {
   long long tiles_used = 0;
   bool join = true;  // make the context stream wait for each run's completion
   std::vector<void *> arenas;  // packed alignments of rnj_batch_add_many, freed by clear
+  int run_alns = 0;           // alignments of the last run: slots below it have a maximum
   std::vector<int> host_max;  // maxima of the last run, read once per run
   bool host_max_valid = false;
   // Launch shape from the tuner: the fused kernel's ring depth of the last run
@@ -98,6 +99,27 @@ void free_batch(rnj_batch *b) {
   if (b->ev_done) cudaEventDestroy(b->ev_done);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
+}
+
+// The maximum of a slot in the last run, 0 for a slot added since.  The maxima of
+// all slots are read once per run: one wait and one copy, and nothing for the other
+// slots (a finished event still cost 1.8 us a slot).
+int slot_max(rnj_batch *b, int slot, float *out) {
+  if (!b->host_max_valid) {
+    DeviceGuard g(b->ctx->device);
+    RNJ_CUDA(cudaEventSynchronize(b->ev_done), "batch sync");
+    b->host_max.assign(b->run_alns, 0);
+    if (b->run_alns > 0) {
+      RNJ_CUDA(cudaMemcpyAsync(b->host_max.data(), b->d_max, sizeof(int) * b->run_alns,
+                               cudaMemcpyDeviceToHost, b->stream),
+               "max copy");
+      RNJ_CUDA(cudaStreamSynchronize(b->stream), "max copy");
+    }
+    b->host_max_valid = true;
+  }
+  const int bits = slot < (int)b->host_max.size() ? b->host_max[slot] : 0;
+  memcpy(out, &bits, sizeof(float));
+  return RNJ_OK;
 }
 
 }  // namespace
@@ -451,6 +473,7 @@ int rnj_batch_run(rnj_batch *b) {
   RNJ_CUDA(cudaEventRecord(b->ev_uploaded, b->stream), "upload event");
   b->uploaded_pending = true;
   b->host_max_valid = false;
+  b->run_alns = 0;
   if (na > 0) {
     // Maxima and flags cleared, the fused kernel over the tensor-core items (a
     // mixed list by each item's descriptor, any other by its own variant, whose
@@ -471,6 +494,7 @@ int rnj_batch_run(rnj_batch *b) {
                                 b->d_ints + 1, sms * 4, b->stream),
              "fix-up kernel");
   }
+  b->run_alns = na;
   RNJ_CUDA(cudaEventRecord(b->ev_done, b->stream), "done event");
   // Later work on the context stream (copies, new packs) sees the results.
   if (b->join) RNJ_CUDA(cudaStreamWaitEvent(ctx->stream, b->ev_done, 0), "join");
@@ -509,19 +533,8 @@ int rnj_batch_output(rnj_batch *b, int slot, float **d_out, size_t *ld, float *m
   if (d_out) *d_out = en.out;
   if (ld) *ld = en.ld;
   if (max_out) {
-    // The maxima of all slots are read once per run: one wait and one copy, and
-    // nothing for the other slots (a finished event still cost 1.8 us a slot).
-    if (!b->host_max_valid) {
-      DeviceGuard g(b->ctx->device);
-      RNJ_CUDA(cudaEventSynchronize(b->ev_done), "batch sync");
-      b->host_max.assign(b->entries.size(), 0);
-      RNJ_CUDA(cudaMemcpyAsync(b->host_max.data(), b->d_max, sizeof(int) * b->entries.size(),
-                               cudaMemcpyDeviceToHost, b->stream),
-               "max copy");
-      RNJ_CUDA(cudaStreamSynchronize(b->stream), "max copy");
-      b->host_max_valid = true;
-    }
-    memcpy(max_out, &b->host_max[slot], sizeof(float));
+    const int rc = slot_max(b, slot, max_out);
+    if (rc != RNJ_OK) return rc;
   }
   return RNJ_OK;
 }
@@ -533,15 +546,9 @@ int rnj_batch_take(rnj_batch *b, int slot, rnj_mat **out) {
   if (!en.owned || !en.out) return set_error(RNJ_ERR_INVALID, "slot output is not owned by the batch");
   DeviceGuard g(b->ctx->device);
   RNJ_CUDA(cudaEventSynchronize(b->ev_done), "batch sync");
-  if (!b->host_max_valid) {
-    b->host_max.assign(b->entries.size(), 0);
-    RNJ_CUDA(cudaMemcpyAsync(b->host_max.data(), b->d_max, sizeof(int) * b->entries.size(),
-                             cudaMemcpyDeviceToHost, b->stream),
-             "max copy");
-    RNJ_CUDA(cudaStreamSynchronize(b->stream), "max copy");
-    b->host_max_valid = true;
-  }
-  const int bits = b->host_max[slot];
+  float largest = 0.0f;
+  const int rc = slot_max(b, slot, &largest);
+  if (rc != RNJ_OK) return rc;
   rnj_mat *m = new rnj_mat();
   m->ctx = b->ctx;
   m->d = en.out;
@@ -549,7 +556,7 @@ int rnj_batch_take(rnj_batch *b, int slot, rnj_mat **out) {
   m->ld = en.ld;
   m->owns = true;  // the matrix now owns the output buffer
   m->has_host_max = true;
-  memcpy(&m->host_max, &bits, sizeof(float));
+  m->host_max = largest;
   en.owned = false;
   en.out = nullptr;
   *out = m;
@@ -584,6 +591,7 @@ int rnj_batch_clear(rnj_batch *b) {
   b->entries.clear();
   b->tiles_used = 0;
   b->host_max_valid = false;
+  b->run_alns = 0;
   return RNJ_OK;
 }
 

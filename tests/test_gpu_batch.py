@@ -125,3 +125,30 @@ def test_batch_capacity_errors(ctx):
     with pytest.raises(RnjError, match="alignments"):
         batch.add(small, "kim")
     assert batch.size() == (2, 2)
+
+
+def test_maximum_of_a_slot_added_after_the_run(ctx):
+    """A slot that the last run did not hold has the maximum 0, whether another
+    slot's was read before or not; a run that holds it gives its own."""
+    from rapidnj_b200 import api, synth
+    s = synth.tree_dna(200, 500, seed=3, mean_branch=0.1)
+    b = api.Batch(ctx, max_alignments=64, max_tiles=4096)
+    alns = [ctx.alignment(s, 0) for _ in range(40)]
+    first = b.add(alns[0], "kim")
+    assert b.max(first) == 0.0  # nothing has run
+    b.run()
+    want = ctx.distance(alns[0], "kim").max
+    assert b.max(first) == want > 0.0
+    late = [b.add(a, "kim") for a in alns[1:]]
+    assert all(b.max(k) == 0.0 for k in late)
+    m = b.take(late[0])
+    assert m.max == 0.0
+    m.close()
+    b.clear()
+    again = [b.add(a, "kim") for a in alns]
+    b.run()
+    b.synchronize()
+    assert all(b.max(k) == want for k in again)
+    b.clear()
+    assert b.max(b.add(alns[0], "kim")) == 0.0
+    b.close()
