@@ -490,7 +490,7 @@ int rnj_batch_run(rnj_batch *b) {
       RNJ_CUDA(launch_count_batch(b->d_descs, b->d_items_pc, b->d_ints + 1, b->d_ints + 2, sms,
                                   EPI_DIST, b->stream),
                "count kernel");
-    RNJ_CUDA(launch_fixup_batch(b->d_descs, b->d_items_tc, b->d_ints + 0, b->d_items_pc,
+    RNJ_CUDA(launch_fixup_batch(b->d_descs, b->d_items_tc, b->d_ints + 0, true, b->d_items_pc,
                                 b->d_ints + 1, sms * 4, b->stream),
              "fix-up kernel");
   }

@@ -237,8 +237,11 @@ int encode_block_map(const Packed &p, CUtensorMap *map);
 // Batched popcount path (rnj_kernels.cu): persistent, atomic item counter.
 cudaError_t launch_count_batch(const AlnDesc *d_descs, const WorkItem *d_items, const int *d_nitems,
                                int *d_counter, int grid, int epi_mode, cudaStream_t s);
+// pairs_a: items_a is a list of the fused kernel's row pairs; else, and items_b
+// always, single tiles.
 cudaError_t launch_fixup_batch(const AlnDesc *d_descs, const WorkItem *items_a, const int *n_a,
-                               const WorkItem *items_b, const int *n_b, int grid, cudaStream_t s);
+                               bool pairs_a, const WorkItem *items_b, const int *n_b, int grid,
+                               cudaStream_t s);
 // Host helpers shared by the single and batched paths (rnj_api.cu).
 // The process-wide wait settings (rnj_set_wait_limit, rnj_test_wait_on_unset_flag)
 // copied into a kernel's parameters.

@@ -803,12 +803,15 @@ __global__ void __launch_bounds__(256, 1)
   }
 }
 
-// Saturation fix-up over every item of a batch whose tile holds a -1.
+// Saturation fix-up over every item of two lists whose tile holds a -1.  pairs_a:
+// the first list is the fused kernel's, of row pairs (WorkItem); otherwise, as the
+// second always, its items are single tiles, whatever kernel counted them.
 __global__ void __launch_bounds__(256) fixup_batch_kernel(const AlnDesc *__restrict__ descs,
                                                           const WorkItem *__restrict__ items_a,
                                                           const int *__restrict__ n_a,
                                                           const WorkItem *__restrict__ items_b,
-                                                          const int *__restrict__ n_b) {
+                                                          const int *__restrict__ n_b,
+                                                          bool pairs_a) {
   const int na = *n_a, nb = *n_b, lane = threadIdx.x & 31;
   // The CTA's items are gridDim.x apart; every warp looks at 32 of them at a time, a
   // lane each, so that the few flagged tiles are found in one round of loads.
@@ -822,7 +825,7 @@ __global__ void __launch_bounds__(256) fixup_batch_kernel(const AlnDesc *__restr
       const int tile = w.tile & ~kPairSingle;
       if (d.out != nullptr) {
         if (d.tile_flags[tile] != 0) first = tile;
-        if (is_tc_kind(d.kind) && !(w.tile & kPairSingle)) {
+        if (pairs_a && at < na && !(w.tile & kPairSingle)) {
           int ti, tj;
           tri_coords(tile, d.nt, ti, tj);  // a row pair: the second row's tile
           const int next = tile + d.nt - ti - 1;
@@ -863,8 +866,9 @@ cudaError_t launch_count_batch(const AlnDesc *d_descs, const WorkItem *d_items, 
 }
 
 cudaError_t launch_fixup_batch(const AlnDesc *d_descs, const WorkItem *items_a, const int *n_a,
-                               const WorkItem *items_b, const int *n_b, int grid, cudaStream_t s) {
-  fixup_batch_kernel<<<grid, 256, 0, s>>>(d_descs, items_a, n_a, items_b, n_b);
+                               bool pairs_a, const WorkItem *items_b, const int *n_b, int grid,
+                               cudaStream_t s) {
+  fixup_batch_kernel<<<grid, 256, 0, s>>>(d_descs, items_a, n_a, items_b, n_b, pairs_a);
   return cudaGetLastError();
 }
 

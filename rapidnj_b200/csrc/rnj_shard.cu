@@ -239,7 +239,8 @@ int rnj_shard_finish(rnj_shard *s, float global_max) {
            "global max upload");
   const int grid = (int)std::min<long long>(nitems, 4LL * ctx->num_sms);
   ctx_mark(ctx, 2, 0);
-  RNJ_CUDA(launch_fixup_batch(s->d_desc, s->d_items, s->d_ints, s->d_items, s->d_ints + 2, grid, st),
+  RNJ_CUDA(launch_fixup_batch(s->d_desc, s->d_items, s->d_ints, s->fused, s->d_items,
+                              s->d_ints + 2, grid, st),
            "fix-up kernel");
   ctx_mark(ctx, 2, 1);
   return read_words(s, nullptr);

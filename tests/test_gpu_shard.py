@@ -100,3 +100,28 @@ def test_sharded_distance_single_process(ctx):
     want, mx = O.distance_matrix(seqs, O.KIMURA, O.DNA)
     assert g == mx
     assert np.array_equal(np.triu(host) + np.triu(host, 1).T, want)
+
+
+@pytest.mark.parametrize("type_,model", [(O.DNA, "kim"), (O.DNA, "jc"), (O.PROTEIN, "kim")])
+@pytest.mark.parametrize("nshards", [1, 3])
+def test_saturated_shards_of_the_two_kernel_form(ctx, type_, model, nshards):
+    """Packed counts and a transform kernel (tc_epilogue 1) count single tiles, not
+    the fused kernel's row pairs: every shard's -1 become twice the global maximum."""
+    from rapidnj_b200 import api, synth
+    n, L = 700, 40
+    seqs = saturating_dna(n, L, 11) if type_ == O.DNA else synth.iid_protein(n, L, seed=11)
+    seqs[5, :] = ord("-")
+    aln = ctx.alignment(seqs, type_)
+    want = ctx.distance(aln, model)
+    ref, top = want.to_numpy(), want.max
+    assert (ref == np.float32(2.0) * np.float32(top)).any()
+    api.tune_set(n, L, "dna" if type_ == O.DNA else "protein", tc_epilogue=1)
+    try:
+        got, g, shards = assemble(ctx, aln, model, nshards)
+    finally:
+        api.tune_clear()
+    assert g == top
+    assert np.array_equal(got, ref)
+    assert not (got == -1.0).any()
+    for sh in shards:
+        sh.close()
