@@ -472,6 +472,8 @@ int rnj_write_matrix_text(const char *path, const char *const *names, const floa
 
 /* Launch parameters of one bucket of inputs: the alphabet (DNA or protein),
  * the counting rules (RNJ_FASTDIST or not), floor(log2 n) and floor(log2 L).
+ * DNA under the -f rules whose letters let it take the fast rules' kernels (see
+ * rnj_aln_from_host) uses their bucket; the -f bucket is that of its bit planes.
  * No counterpart in the reference (its CPU code has nothing to tune).  The
  * tile edge itself is fixed at 128 pairs: the tensor-core MMA is 128 rows
  * (M = 128) and three 128-column f32 accumulators fill the 512 columns of

@@ -380,7 +380,8 @@ int pack_from_device_chars(rnj_ctx *ctx, const uint8_t *d_chars, int n, int L, s
 
 size_t packed_layout(Packed &p, int n, int L, int type, int flags, int kind, const uint8_t *lut,
                      bool tuned_kernel) {
-  const bool tc_choice = !tuned_kernel || tune_lookup(n, L, type, flags).dna_kernel == 0;
+  const bool tc_choice =
+      !tuned_kernel || tune_lookup(n, L, type, tune_flags(kind, flags)).dna_kernel == 0;
   p.n = n;
   p.L = L;
   p.type = type;
@@ -501,7 +502,7 @@ namespace {
 int run_tc_single(rnj_ctx *ctx, const Packed &p, const EpiParams &ep, int epi_mode) {
   const int nt = tiles_of(p.n);
   const long long ntiles = ep.full ? (long long)nt * nt : tri_tiles(nt);
-  const TuneParams tp = tune_lookup(p.n, p.L, p.type, p.flags);
+  const TuneParams tp = tune_for(p);
   AlnDesc d = desc_for(p, ep);
   d.band = tp.tile_band;
   if (epi_mode != EPI_COUNTS && tc_fused_form(p, tp))
@@ -580,7 +581,7 @@ int run_popcount(rnj_ctx *ctx, const Packed &p, int ckind, int nk, int nt, EpiPa
   // K split (tuned per bucket): short triangles of long alignments leave most
   // SMs idle with one CTA per tile; splitting the columns over several CTAs
   // per tile (atomic count accumulation, then the transform) fills them.
-  const TuneParams tp = tune_lookup(p.n, p.L, p.type, p.flags);
+  const TuneParams tp = tune_for(p);
   ep.stages = tp.pop_stages;
   const bool split = tp.ksplit > 1 && nk >= 2 && !ep.full &&
                      (size_t)p.n * p.n * 3 * sizeof(uint32_t) <= (size_t)1 << 30;

@@ -417,7 +417,7 @@ int rnj_batch_run(rnj_batch *b) {
     for (int a = 0; a < na; ++a) {
       const Packed &p = b->entries[a].aln->p;
       bool found = false;
-      const TuneParams tp = tune_lookup(p.n, p.L, p.type, p.flags, &found);
+      const TuneParams tp = tune_for(p, &found);
       tuned += found ? 1 : 0;
       bands[a] = tp.tile_band > 0 ? tp.tile_band : kBand;
       const long long work = b->entries[a].ntiles * cost(a);

@@ -201,7 +201,7 @@ static int tc_tiles(rnj_ctx *ctx, const Packed &p, int model, const F64Params &f
   const int chunk = (int)std::min<long long>(ntiles, kTcChunkTiles);
   int rc = ensure_packed(ctx, chunk);
   if (rc != RNJ_OK) return rc;
-  const TuneParams tp = tune_lookup(p.n, p.L, p.type, p.flags);
+  const TuneParams tp = tune_for(p);
   AlnDesc d = desc_for(p, ctx_epi(ctx, p, model));
   d.band = tp.tile_band;
   if ((rc = encode_block_map(p, &d.map)) != RNJ_OK) return rc;

@@ -161,6 +161,15 @@ struct TuneParams {
 // table (filled by rnj_tune / rnj_tune_load / RNJ_TUNE_CACHE) holds one, else
 // the defaults (*found, when given, says which).
 TuneParams tune_lookup(int n, int L, int type, int flags, bool *found = nullptr);
+// Those of a packed alignment: the bucket of the kernels that its layout runs.  DNA
+// under the naive rules whose letters let it take the fast rules' layouts (rnj_api.cu)
+// runs the fast rules' kernels; the naive bucket's choices are those of its bit planes.
+inline int tune_flags(int kind, int flags) {
+  return kind == KIND_DNA || kind == KIND_DNA_TC ? flags | RNJ_FASTDIST : flags;
+}
+inline TuneParams tune_for(const Packed &p, bool *found = nullptr) {
+  return tune_lookup(p.n, p.L, p.type, tune_flags(p.kind, p.flags), found);
+}
 
 // One alignment of a batched pack (rnj_batch_add_many): the multi-alignment
 // pack kernels take an array of these and find the alignment of each work unit

@@ -112,7 +112,7 @@ extern "C" int rnj_distance_rows(rnj_ctx *ctx, rnj_aln *aln, int model, int band
   EpiParams ep = ctx_epi(ctx, p, model);
   ep.full = 1;
   ep.ld = (size_t)n;
-  const TuneParams tp = tune_lookup(p.n, p.L, p.type, p.flags);
+  const TuneParams tp = tune_for(p);
   ep.stages = tp.pop_stages;
 
   RowBuffers buf(ctx);

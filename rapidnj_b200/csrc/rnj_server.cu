@@ -387,7 +387,7 @@ void prepare_all(rnj_server *s, const std::vector<Request *> &reqs) {
       e = cudaMemcpyAsync(s->d_descs + slot, s->h_descs + slot, sizeof(AlnDesc),
                           cudaMemcpyHostToDevice, ctx->stream);
     }
-    const TuneParams tp = tune_lookup(p.n, p.L, p.type, p.flags);
+    const TuneParams tp = tune_for(p);
     if (e == cudaSuccess)
       e = launch_live_publish(s->live, slot, nt, tp.tile_band, first, ntiles, s->d_max + slot,
                               s->d_flags + first, ctx->stream);

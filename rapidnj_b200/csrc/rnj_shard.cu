@@ -143,7 +143,7 @@ int rnj_shard_create(rnj_ctx *ctx, rnj_aln *aln, int model, int shard, int nshar
   s->owns_out = (d_out == nullptr);
   s->ld = d_out ? ld : (size_t)std::max(4, (p.n + 3) / 4 * 4);
   s->out = d_out;
-  s->tp = tune_lookup(p.n, p.L, p.type, p.flags);
+  s->tp = tune_for(p);
   s->fused = is_tc_kind(p.kind) && tc_fused_form(p, s->tp);
   std::vector<WorkItem> items;
   if (s->fused) pair_items_of_range(0, tiles_of(p.n), t0, t1, items);

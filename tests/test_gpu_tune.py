@@ -131,3 +131,36 @@ def test_k_split_helps_few_long_sequences(ctx):
     # splitting the columns is faster.
     p = ctx.tune(256, 20000, "protein", popcount=True)
     assert p.ksplit > 1
+
+
+@pytest.mark.parametrize("letters,bucket", [("upper", True), ("lower", False)])
+def test_naive_rules_use_the_bucket_of_the_kernel_that_runs(ctx, letters, bucket):
+    """-f DNA whose letters send it to the tensor cores takes the fast rules' entry,
+    any other the -f entry; the matrix is the untuned one either way."""
+    n, L = 300, 2000
+    seqs = synth.tree_dna(n, L, seed=5)
+    if letters == "lower":
+        seqs = np.char.lower(seqs.view("S1")).view(np.uint8)
+
+    def run():
+        b = api.Batch(ctx, max_alignments=1, max_tiles=64)
+        aln = ctx.alignment(seqs, "dna", fastdist=False)
+        slot = b.add(aln, "kim")
+        b.run()
+        b.synchronize()
+        m = b.take(slot)
+        got, shape = (m.to_numpy(), m.max), b.tuning()
+        m.close()
+        b.close()
+        one = ctx.distance(aln, "kim")
+        same((one.to_numpy(), one.max), got)
+        return got, shape
+
+    ref, shape = run()
+    assert shape == (6, 0)
+    for fast in (True, False):
+        api.tune_clear()
+        api.tune_set(n, L, "dna", fastdist=fast, tc_stages=3, ksplit=2)
+        got, shape = run()
+        same(got, ref)
+        assert shape == ((3 if bucket else 6, 1) if fast == bucket else (6, 0))
