@@ -877,6 +877,16 @@ __device__ __forceinline__ void pair_produce(const TcShared &sh, int rank, const
       }
     }
   }
+  // The leader's commits arrive on the stages' barriers of both CTAs, and nothing else
+  // waits for those of the last round of the ring: a CTA leaves after them.  (They are
+  // long past when the epilogue ends.  A stage never used passes at once.)
+  for (int k = 0; good && k < sh.nst; ++k) {
+    good = tc_wait(&sh.empty_bar[s], pph ^ 1u, sh.abort_flag, limit);
+    if (++s == sh.nst) {
+      s = 0;
+      pph ^= 1u;
+    }
+  }
   if (!good) pair_abort(sh);
   *sh.issued = issued;
 }

@@ -102,3 +102,27 @@ def test_column_slices(ctx, typ, model, wrap, n):
     assert np.array_equal(out[:, :n].cpu().numpy().view(np.int32), want.view(np.int32))
     assert np.float32(mx) == np.float32(with_batch.max(slot))
     assert bool((out[:, n:] == -7.0).all())
+
+
+@pytest.mark.parametrize("residues", [1, 2, 3, 4, 9])
+@pytest.mark.parametrize("L", [100, 600])
+@pytest.mark.parametrize("depth", [0, 3])
+def test_fewer_and_more_stages_than_the_ring(ctx, residues, L, depth):
+    """1 + residues feature blocks of one or two stages each, from half a ring to
+    several rounds of it, with one and several items a pair of CTAs."""
+    from rapidnj_b200 import api
+    letters = np.frombuffer(b"ARNDCQEGH", np.uint8)[:residues]
+    rng = np.random.default_rng(residues + L)
+    for n in (5, 300, 2300):
+        s = letters[rng.integers(0, residues, (n, L))]
+        s[rng.random((n, L)) < 0.05] = ord("-")
+        if depth:
+            api.tune_set(n, L, "protein", tc_stages=depth)
+        try:
+            fused = ctx.distance(ctx.alignment(s, 1), "kim")
+            got, mx = fused.to_numpy(), fused.max
+        finally:
+            api.tune_clear()
+        planes = ctx.distance(ctx.alignment(s, 1, popcount=True), "kim")
+        assert np.array_equal(got.view(np.int32), planes.to_numpy().view(np.int32))
+        assert mx == planes.max
