@@ -320,10 +320,10 @@ int rnj_batch_output(rnj_batch *batch, int slot, float **d_out, size_t *ld, floa
 /* Moves a batch-allocated output into a matrix handle (for rnj_mat_copy_rows). */
 int rnj_batch_take(rnj_batch *batch, int slot, rnj_mat **out);
 int rnj_batch_size(rnj_batch *batch, int *alignments, long long *tiles);
-/* The launch shape of the last run: the tensor-core ring depth it ran with
- * (the tuned depth of the bucket holding most of its work) and how many of its
- * alignments had a tuned entry (each one's tile-order band comes from it).
- * Either pointer may be NULL. */
+/* The launch shape of the last run: its tensor-core ring depth as in
+ * rnj_tune_params::tc_stages (the tuned depth of the bucket holding most of its
+ * work, 6 without one) and how many of its alignments had a tuned entry (each
+ * one's tile-order band comes from it).  Either pointer may be NULL. */
 int rnj_batch_tuning(rnj_batch *batch, int *ring_depth, int *tuned_alignments);
 /* Forgets the alignments (frees outputs still owned by the batch). */
 int rnj_batch_clear(rnj_batch *batch);
@@ -491,8 +491,11 @@ typedef struct rnj_tune_params {
   int tc_epilogue;     /* tensor cores: 0 the exact transform in the counting kernel's own
                           epilogue warps (one launch), 1 packed counts and a separate
                           transform kernel at higher occupancy */
-  int tc_stages;       /* tensor cores: shared-memory ring depth in 256-column K blocks,
-                          2..6 fused, 2..7 two-kernel (0 = the deepest) */
+  int tc_stages;       /* tensor cores: shared memory of the operand ring in 32 KB (a
+                          256-column K block of two 128-row tiles), 0 = the deepest.
+                          Two-kernel and served form: that many stages, 2..7 and 2..6.
+                          Fused: 2/3 as many stages, of 48 KB, in each CTA of a pair:
+                          6 (the deepest) four, 5 three, 4 and below two */
   int pop_stages;      /* bit-plane kernel: ring depth in 256-site K blocks, raised to the
                           3 (DNA, 2-bit codes) or 2 (5- and 7-bit codes) its distance
                           staging needs; 0 = the deepest, 4 (DNA, 2-bit) or 3 */

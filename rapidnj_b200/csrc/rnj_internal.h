@@ -278,7 +278,7 @@ cudaError_t launch_tc_transform(const AlnDesc *d_descs, const WorkItem *d_items,
 // flags.  Every alignment has at most kMaxFusedColumns columns.
 // variant: the transform of every item (fused_variant_for), or FUSED_ANY to
 // choose per item from its descriptor.  stages: the ring depth (0: the default, 6;
-// the tuner's tc_stages).  d_descs null: the one descriptor is `one` (host), which
+// the tuner's tc_stages; in 32 KB, see kFusedRings).  d_descs null: the one descriptor is `one` (host), which
 // goes along with the launch.
 enum FusedVariant {
   FUSED_K2P = 0, FUSED_JC = 1, FUSED_PROTEIN = 2, FUSED_GENERIC = 3, FUSED_FULL = 4, FUSED_ANY = 5
@@ -292,8 +292,11 @@ cudaError_t launch_tc_fused(const AlnDesc *d_descs, const WorkItem *d_items, int
 long long pair_items(int nt);  // items of a whole triangle of nt tile rows
 void pair_items_of_band(int aln, int nt, int r0, int r1, std::vector<WorkItem> &out);
 void pair_items_of_range(int aln, int nt, long long t0, long long t1, std::vector<WorkItem> &out);
-// The ring depth launch_tc_fused runs with for a requested `stages`.
+// The depth a requested `stages` stands for: that number within 2 .. 6, 6 for 0.
 int fused_ring_depth(int stages);
+// The depths at which launch_tc_fused runs a ring of its own, the default first: four,
+// three and two stages of 48 KB (rnj_tcf.cu); 2 and 3 run the ring of 4.
+constexpr int kFusedRings[] = {6, 5, 4};
 
 // The live work list of the served form (rnj_server.cu): triangle tiles of
 // tensor-core alignments appended while tc_live_kernel runs.  The publisher

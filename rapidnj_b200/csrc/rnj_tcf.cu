@@ -83,12 +83,22 @@ constexpr size_t kTcfSmemBytes = tc_smem_bytes(kPairStages, kTcfExtra, kPairStag
 static_assert(kTcfSmemBytes <= 232448, "fits the shared memory of one CTA");
 static_assert(sizeof(c_pam.dist) <= kTcfPamBytes, "the Dayhoff distances fit their slot");
 
-// Stages of the pair form in the ring of a requested depth (0: the default).
+// Stages of the pair form in the ring of a requested depth (0: the default): stages
+// of 48 KB in that many times 32 KB, at least two, so that 6 gives 4, 5 gives 3 and
+// 4, 3 and 2 the same 2.
 __host__ __device__ constexpr int pair_stages(int depth) {
   const int st = tc_ring_depth(depth, kTcfStages, kTcfStages) * 2 / 3;
   return st < kTcMinStages ? kTcMinStages : st;
 }
 static_assert(pair_stages(0) == kPairStages, "the deepest ring");
+// kFusedRings: the depths that differ, deepest first.
+constexpr bool every_ring_once() {
+  int st = kPairStages;
+  for (const int depth : kFusedRings)
+    if (pair_stages(depth) != st--) return false;
+  return st == kTcMinStages - 1;
+}
+static_assert(every_ring_once(), "each ring of the pair form has one depth in the list");
 
 // The tables (ln: this lane's copy) and this warp's transpose buffer.
 struct TcfTables {

@@ -425,7 +425,8 @@ extern "C" int rnj_tune(rnj_ctx *ctx, int n, int L, int type, int flags, rnj_tun
       if ((rc = consider(c, false)) != RNJ_OK) break;
     }
     const int band = best.tile_band;
-    for (int st : {5, 4, 3}) {
+    for (int st : kFusedRings) {
+      if (st == kFusedRings[0]) continue;  // the default, timed with the bands
       if (rc != RNJ_OK || !fused_ok) break;
       rnj_tune_params c = base;
       c.tile_band = band;
