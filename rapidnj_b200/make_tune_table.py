@@ -10,7 +10,10 @@ every bucket the standard workloads touch:
   bucket clipped to the range.
 
 A bucket is (alphabet, counting rules, floor(log2 N), floor(log2 L)); every
-choice in it gives the same distances, only the time differs.  Usage:
+choice in it gives the same distances, only the time differs.  The fused kernel's
+ring depth is left at its default: no shallower ring was faster by more than the
+runs of one depth differ, and a batch runs all its alignments with the depth of
+one of them.  Usage:
 
     python -m rapidnj_b200.make_tune_table [--out PATH] [--device N]
 
@@ -67,6 +70,9 @@ def main(argv=None):
     t0 = time.time()
     for k, (n, L, t) in enumerate(shapes):
         p = ctx.tune(n, L, t)
+        if p.tc_epilogue == 0 and p.tc_stages != 0:
+            p.tc_stages = 0
+            api.tune_set(n, L, t, **p.as_dict())
         print(f"[{k + 1}/{len(shapes)}] {t} {n} x {L}: {p.as_dict()}", flush=True)
     api.tune_save(args.out)
     ctx.close()

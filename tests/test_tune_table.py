@@ -160,3 +160,33 @@ def test_shipped_table_beside_the_library(tmp_path):
     assert run() == ["0", "8", "5"]
     assert run(RNJ_NO_TUNE_TABLE="1")[0] != "0"
     assert run(RNJ_TUNE_CACHE=str(other)) == ["0", "24", "3"]
+
+
+def test_the_shipped_table_is_what_its_generator_writes(tmp_path, monkeypatch):
+    """Whatever ring depth the tuner stores for the fused kernel, the generator
+    writes the default; other choices and the two-kernel form's depth stay."""
+    from rapidnj_b200 import make_tune_table
+
+    class Tuner:
+        def __init__(self, device):
+            pass
+
+        def tune(self, n, L, type_):
+            two = type_ == "protein"
+            api.tune_set(n, L, type_, tile_band=8, tc_epilogue=int(two), tc_stages=5 if two else 4,
+                         ms=0.5)
+            return api.tune_get(n, L, type_)
+
+        def close(self):
+            pass
+
+    monkeypatch.setattr(api, "Context", Tuner)
+    path = tmp_path / "table.txt"
+    make_tune_table.main(["--out", str(path)])
+    made = [x.split() for x in path.read_text().splitlines() if not x.startswith("#")]
+    shipped = open(os.path.join(ROOT, "rapidnj_b200", "tune_b200.txt")).read().splitlines()
+    shipped = [x.split() for x in shipped if not x.startswith("#")]
+    assert {tuple(x[:4]) for x in made} == {tuple(x[:4]) for x in shipped}
+    assert {(x[0], x[6], x[9], x[10]) for x in made} == {("dna", "8", "0", "0"),
+                                                         ("protein", "8", "1", "5")}
+    assert all(x[10] == "0" for x in shipped if x[9] == "0")
