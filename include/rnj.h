@@ -126,7 +126,8 @@ int rnj_probe_int_peaks(rnj_ctx *ctx, double *popc_per_s, double *lop3_per_s);
 int rnj_probe_tc_peak(rnj_ctx *ctx, double *fp4_flops_per_s);
 /* Self-check of the fused epilogue's quotients on the device, against
  * correctly rounded division: the float quotients by the valid count (the
- * reference's (float)((double)num / (double)n)) for every 0 <= num <= n < 2^16,
+ * reference's (float)((double)num / (double)n)) for every 0 <= num <= n < 2^16, with
+ * the numerator as it is and as the K2P epilogue scales it (by 2 and by 4),
  * and JC's (double)p / b for every float p in [0, 1] and b = 3/4, 19/20.
  * *mismatches is 0 on a sound build.  No counterpart in the reference. */
 int rnj_check_quotient16(rnj_ctx *ctx, unsigned long long *mismatches);

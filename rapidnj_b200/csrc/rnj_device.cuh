@@ -375,36 +375,6 @@ __device__ __forceinline__ float k2p_distance(unsigned long long ts_count,
   return k2p_two_logs(a, b);
 }
 
-// 1 / d for an integer 1 <= d < 2^16 given as a float: one Newton-Raphson step
-// r0 + r0 (1 - d r0) from the fast reciprocal (|d r0 - 1| <= 2^-21).  1 - d r0
-// is exact as a fused multiply-add (d r0 has at most 40 significant bits and
-// lies within 2^-21 of 1; the difference is a multiple of 2^-39), so the
-// result has |d y - 1| <= 2^-42 + 2^-24 < 2^-23.9.
-__device__ __forceinline__ float recip16(float d) {
-  const float r0 = rcp_approx(d);
-  return __fmaf_rn(r0, __fmaf_rn(-d, r0, 1.0f), r0);
-}
-
-// fl32(num / d) for integers 0 <= num <= d < 2^16 (d as a float, y = recip16(d))
-// in float arithmetic.  q0 = fl(num y) is within 2^-22.9 (relative) of num / d;
-// the residual num - d q0 is a multiple of ulp(q0) with fewer than 2^17 of them,
-// so one fused multiply-add gives it exactly; q = fl(q0 + r y), one more fused
-// multiply-add, rounds num / d + (num / d - q0)(d y - 1), which is within
-// 2^-22 ulp of num / d.  num / d lies at least 2^-18 ulp from every float
-// midpoint (a midpoint is M 2^-e with M odd of 25 bits, and num / d = M 2^-e
-// would need M | num < 2^16), so q is the correctly rounded quotient: the
-// reference's (float)((double)num / (double)d) and (float)num / (float)d (the
-// double quotient is no midpoint either, so its float rounding agrees).
-// A numerator scaled by a power of two gives the quotient scaled by it (every
-// step commutes with the scale), which the fused epilogue uses for 4 P and 2 Q.
-__device__ __forceinline__ float quotient_of(float fnum, float d, float y) {
-  const float q0 = __fmul_rn(fnum, y);
-  return __fmaf_rn(__fmaf_rn(-q0, d, fnum), y, q0);
-}
-__device__ __forceinline__ float quotient16(uint32_t num, float d, float y) {
-  return quotient_of(__fsub_rn(__uint_as_float(0x4B000000u | num), 8388608.0f), d, y);
-}
-
 // Two floats in one 64-bit register, and the packed operations on them (each
 // half rounded like the scalar operation): the float part of the fused epilogue
 // takes two pairs at a time.
@@ -432,13 +402,32 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-// recip16 and quotient_of for two pairs; nd = -d.
+
+// 1 / d for integers 1 <= d < 2^16 given as floats (nd = -d): one Newton-Raphson step
+// r0 + r0 (1 - d r0) from the fast reciprocal (|d r0 - 1| <= 2^-21).  1 - d r0
+// is exact as a fused multiply-add (d r0 has at most 40 significant bits and
+// lies within 2^-21 of 1; the difference is a multiple of 2^-39), so the
+// result has |d y - 1| <= 2^-42 + 2^-24 < 2^-23.9.
 __device__ __forceinline__ f32x2 recip16_2(f32x2 d, f32x2 nd) {
   float a, b;
   unpack2(d, a, b);
   const f32x2 r0 = pack2(rcp_approx(a), rcp_approx(b));
   return fma2(r0, fma2(nd, r0, pack2(1.0f, 1.0f)), r0);
 }
+
+// fl32(num / d) for integers 0 <= num <= d < 2^16 (nd = -d, y = recip16_2(d, nd))
+// in float arithmetic.  q0 = fl(num y) is within 2^-22.9 (relative) of num / d;
+// the residual num - d q0 is a multiple of ulp(q0) with fewer than 2^17 of them,
+// so one fused multiply-add gives it exactly; q = fl(q0 + r y), one more fused
+// multiply-add, rounds num / d + (num / d - q0)(d y - 1), which is within
+// 2^-22 ulp of num / d.  num / d lies at least 2^-18 ulp from every float
+// midpoint (a midpoint is M 2^-e with M odd of 25 bits, and num / d = M 2^-e
+// would need M | num < 2^16), so q is the correctly rounded quotient: the
+// reference's (float)((double)num / (double)d) and (float)num / (float)d (the
+// double quotient is no midpoint either, so its float rounding agrees).
+// A numerator scaled by a power of two gives the quotient scaled by it (every
+// step commutes with the scale), which the fused epilogue uses for 4 P and 2 Q.
+// rnj_check_quotient16 runs both functions over all of these.
 __device__ __forceinline__ f32x2 quotient_of_2(f32x2 num, f32x2 nd, f32x2 y) {
   const f32x2 q0 = mul2(num, y);
   return fma2(fma2(q0, nd, num), y, q0);

@@ -138,17 +138,28 @@ extern "C" int rnj_probe_tc_peak(rnj_ctx *ctx, double *fp4_flops_per_s) {
 namespace rnj {
 
 // Every (num, d) with 1 <= d < 2^16 and 0 <= num <= d (block d, threads over
-// num): quotient16 against the correctly rounded float division and against
-// the reference's double division rounded to float; mismatches counted.
+// num, a pair num and d - num at a time), the numerator as it is, doubled and
+// quadrupled: the fused epilogue's recip16_2 and quotient_of_2 against the correctly
+// rounded float division and against the reference's double division rounded to
+// float, scaled alike; mismatches counted.
 __global__ void __launch_bounds__(256) quotient16_check_kernel(unsigned long long *mismatches) {
   const uint32_t d = blockIdx.x + 1;
-  const float fd = (float)d, y = recip16(fd);
+  const float fd = (float)d;
+  const f32x2 dd = pack2(fd, fd), nd = pack2(-fd, -fd), y = recip16_2(dd, nd);
   unsigned long long bad = 0;
-  for (uint32_t num = threadIdx.x; num <= d; num += blockDim.x) {
-    const float q = quotient16(num, fd, y);
-    const float f = __fdiv_rn((float)num, fd);
-    const float g = __double2float_rn(__ddiv_rn((double)num, (double)d));
-    bad += (__float_as_uint(q) != __float_as_uint(f)) + (__float_as_uint(q) != __float_as_uint(g));
+  for (uint32_t num = threadIdx.x; num <= d / 2; num += blockDim.x) {
+    const uint32_t n2[2] = {num, d - num};
+    for (float scale = 1.0f; scale <= 4.0f; scale *= 2.0f) {
+      float q[2];
+      unpack2(quotient_of_2(pack2(scale * (float)n2[0], scale * (float)n2[1]), nd, y), q[0], q[1]);
+      for (int k = 0; k < 2; ++k) {
+        const float f = __fmul_rn(scale, __fdiv_rn((float)n2[k], fd));
+        const float g =
+            __fmul_rn(scale, __double2float_rn(__ddiv_rn((double)n2[k], (double)d)));
+        bad += (__float_as_uint(q[k]) != __float_as_uint(f)) +
+               (__float_as_uint(q[k]) != __float_as_uint(g));
+      }
+    }
   }
   if (bad) atomicAdd(mismatches, bad);
 }
@@ -173,7 +184,7 @@ __global__ void __launch_bounds__(256) jc_quotient_check_kernel(unsigned long lo
 }  // namespace rnj
 
 // The fused epilogue's quotients over their whole domain: the float quotients
-// (quotient16) and the JC double quotients (div_by_b).
+// (quotient_of_2) and the JC double quotients (div_by_b).
 extern "C" int rnj_check_quotient16(rnj_ctx *ctx, unsigned long long *mismatches) {
   if (!ctx || !mismatches) return set_error(RNJ_ERR_INVALID, "null argument");
   void *sv = nullptr;

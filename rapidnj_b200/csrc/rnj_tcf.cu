@@ -18,7 +18,7 @@
 //   * it computes the distances of each lane from the f32 sums as they are,
 //     eight pairs at a time without branches: exact sums and differences, the
 //     quotients by the valid count in float (the same floats as the reference's
-//     divisions, quotient_of), a and b in double, the logarithm from a
+//     divisions, quotient_of_2), a and b in double, the logarithm from a
 //     table in shared memory (neg_quarter_ln) and the rounding check
 //     (RoundCheck), while the tensor cores already count the next tile;
 //   * stores: the mirror entries out[j][i] as coalesced 128-byte row segments

@@ -179,3 +179,18 @@ def test_float_quotient_of_16_bit_counts():
                     continue
                 want = f32(Fraction(num, d))
                 assert quotient16(num, d, ulps) == want, (num, d, ulps)
+
+
+def test_scaled_numerators_scale_the_quotient():
+    """The fused epilogue forms 4 P / n and 2 Q / n: every step commutes with the
+    power of two."""
+    rng = np.random.default_rng(17)
+    for d in [1, 2, 3, 79, 65535] + [int(x) for x in rng.integers(4, 1 << 16, 40)]:
+        for num in {0, 1, d - 1, d} | set(int(x) for x in rng.integers(0, d + 1, 12)):
+            for ulps in (-4, 0, 4):
+                r0 = seed(d, ulps)
+                y = fma32(r0, fma32(-float(d), r0, 1.0), r0)
+                for scale in (2, 4):
+                    q0 = f32(np.float32(scale * num) * np.float32(y))
+                    q = fma32(fma32(-q0, float(d), float(scale * num)), y, q0)
+                    assert q == scale * f32(Fraction(num, d)), (num, d, ulps, scale)
