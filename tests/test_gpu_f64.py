@@ -139,3 +139,43 @@ def test_tiles_and_passes(ctx, n, L, typ, model):
     d = (m.abs().float().view(torch.int32) - flt.abs().view(torch.int32)).abs()
     assert int(d.max()) <= 1 and int((d == 1).sum()) <= max(2, 1e-6 * n * n)
     assert mx <= float(m.max())
+
+
+@pytest.mark.parametrize("n,L", [(31, 40), (129, 300), (641, 100), (12000, 64)])
+@pytest.mark.parametrize("typ,model", [(0, "kim"), (0, "jc"), (1, "kim")])
+@pytest.mark.parametrize("popcount", [False, True])
+def test_the_maximum_is_the_matrix_maximum(ctx, n, L, typ, model, popcount):
+    from rapidnj_b200 import synth
+    # The largest distance is one of the last rows' (of DNA that of two of them, in the
+    # last tile) and so is the one saturated pair: in the last column of tiles and the
+    # last pass (12,000 rows take two passes of packed counts).  The maximum is the
+    # matrix's, and twice it replaces the pair's -1.
+    if n > 1000 and (popcount or model == "jc"):
+        pytest.skip("one model and layout at the large size")
+    letters = np.frombuffer(b"AGTC" if typ == 0 else b"ARNDCQEGHILKMFPSTWYV", np.uint8)
+    s = (synth.tree_dna if typ == 0 else synth.tree_protein)(min(n, 700), L, seed=n,
+                                                             mean_branch=0.003)
+    s = np.ascontiguousarray(s[np.arange(n) % s.shape[0]])
+    other = np.arange(256, dtype=np.uint8)
+    other[letters] = np.roll(letters, len(letters) // 2)
+    k = L // 5
+    s[n - 5:] = s[0]
+    s[n - 5, :k] = other[s[n - 5, :k]]
+    s[n - 4, -k:] = other[s[n - 4, -k:]]
+
+    def call():
+        m, mx = ctx.distance_f64(ctx.alignment(s, typ, popcount=popcount), model)
+        ctx.synchronize()
+        return m, mx
+
+    m, mx = call()
+    assert mx > 0.0 and mx == float(m.max())
+    assert mx == float(m[n - 5, n - 4] if typ == 0 else m[:, n - 5:n - 3].max())
+    if model == "jc":
+        return  # no common site is distance 0 there
+    s[n - 2, : L // 2] = ord("-")
+    s[n - 1, L // 2:] = ord("-")
+    m, mx2 = call()
+    assert float(m[n - 2, n - 1]) == float(m[n - 1, n - 2]) == 2.0 * mx2
+    m[n - 2, n - 1] = m[n - 1, n - 2] = 0.0
+    assert mx2 == float(m.max())
