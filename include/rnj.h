@@ -68,7 +68,9 @@ enum {
    * counted on the tensor cores by default (tcgen05 kind::mxf4: FP4 features in
    * {-1, 0, +1} with unit block scales, exact f32 sums).  This flag selects the
    * bit-plane popcount kernels instead: same counts, far fewer bytes of packed
-   * input per site.  DNA with the -f rules always uses the popcount kernels. */
+   * input per site.  DNA with the -f rules (no RNJ_FASTDIST) uses the bit planes,
+   * except where rnj_aln_from_host's packing finds letters that both rules count
+   * alike; with this flag it always does. */
   RNJ_POPCOUNT = 8
 };
 
@@ -143,7 +145,14 @@ int rnj_detect_type(const char *seq0, int L);
  * dataloaderFasta.hpp:135-182) and storeDataDNA_gpu (KimuraDistance.cpp:19).
  * `type` RNJ_UNKNOWN detects it from seqs[0].  `flags` is RNJ_FASTDIST |
  * RNJ_COMPAT_PROTEIN_WRAP | RNJ_FULL_ROWS.  Bytes are the characters of the
- * alignment as the reference's parsers keep them (33..126). */
+ * alignment as the reference's parsers keep them (33..126).
+ * This call and the next two synchronise the context's stream where the layout
+ * depends on the bytes: protein, whose residues are ranked, and DNA under the -f
+ * rules from 1,536 columns or 2,560 sequences on (without RNJ_FULL_ROWS and
+ * RNJ_POPCOUNT, and not while the stream is captured).  Such DNA takes the fast
+ * rules' layout, for the tensor cores, unless it holds a lower-case a, c, g or t or
+ * a U of either case, which the two rules count differently: then the bit planes,
+ * 15 to 20 us later than without the look at the bytes. */
 int rnj_aln_from_host(rnj_ctx *ctx, const char *const *seqs, int n, int L, int type,
                       int flags, rnj_aln **out);
 /* Same, from one host buffer of n rows with stride ld >= L. */
@@ -284,8 +293,10 @@ int rnj_distance_matrix_host_ex(rnj_ctx *ctx, const char *chars, int n, int L, s
 
 /* Many alignments computed together.  The triangle tiles of every alignment
  * added form one device work list, ordered by decreasing cost, that one
- * persistent launch per kernel family consumes (the tensor-core kernel for DNA,
- * the bit-plane kernel for -f alignments and large alphabets), followed by the
+ * persistent launch per kernel family consumes (the tensor-core kernel or the
+ * bit-plane kernel, by the layout each alignment is packed in; rnj_batch_add_many
+ * packs DNA under the -f rules, and proteins of more than 31 distinct residues, in
+ * bit planes), followed by the
  * saturation fix-up; a run uploads the descriptors and work lists that these
  * read.  For a stream of alignments this replaces one driver call per
  * alignment (JCdistance / KimuraDistance per input, or per bootstrap replicate

@@ -333,8 +333,11 @@ namespace {
 // row's case).  The plane kernel, with a population count per word and pair, then
 // gives way to the tensor cores: 3,001 x 4,003 sites 880 -> 105 us, 500 x 2,000 191 ->
 // 45, 3,000 x 60 214 -> 82.  Letters that need the planes cost the call the scan and
-// its wait, 16 us, so the scan is kept to where the planes take 150 us or more: many
-// columns (60 us + 0.06 a column, whatever the rows) or many rows.  Under stream
+// its wait, 15 to 20 us (16 x 1,536 sites 121 -> 136, 500 x 2,000 194 -> 210, 3,001 x
+// 4,003 894 -> 914), so the scan is kept to where the planes take 120 us or more: many
+// columns (60 us + 0.06 a column, whatever the rows) or many rows.  (Planes packed
+// behind the scan while the host waits: 11 to 14 us in place of these, but upper-case
+// 3,001 x 4,003 sites 126 -> 141 us.)  Under stream
 // capture there is no waiting for the scan; whole rows (FULL_ROWS) and calls that ask
 // for the planes stay with them.
 bool naive_scan_pays(rnj_ctx *ctx, int n, int L, int flags) {

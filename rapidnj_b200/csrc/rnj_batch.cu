@@ -1,8 +1,8 @@
 // rnj_batch.cu -- many alignments in one pass: a device work list of the
 // triangle tiles of every alignment in the batch, ordered by decreasing cost,
 // consumed by one persistent launch per kernel family (the tcgen05 kernel for
-// DNA, the bit-plane kernel for protein and -f alignments) and a fix-up over the
-// flagged tiles.  A run uploads the descriptors and work lists and launches the
+// alignments packed as features, the bit-plane kernel for the others: -f DNA packed
+// here, large alphabets) and a fix-up over the flagged tiles.  A run uploads the descriptors and work lists and launches the
 // kernels that have items.
 #include <cuda_runtime.h>
 #include <stdint.h>
