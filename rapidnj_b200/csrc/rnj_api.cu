@@ -336,7 +336,7 @@ namespace {
 // its wait, 15 to 20 us (16 x 1,536 sites 121 -> 136, 500 x 2,000 194 -> 210, 3,001 x
 // 4,003 894 -> 914), so the scan is kept to where the planes take 120 us or more: many
 // columns (60 us + 0.06 a column, whatever the rows) or many rows.  (Planes packed
-// behind the scan while the host waits: 11 to 14 us in place of these, but upper-case
+// behind the scan while the host waits: 11 to 15 us in place of these, but upper-case
 // 3,001 x 4,003 sites 126 -> 141 us.)  Under stream
 // capture there is no waiting for the scan; whole rows (FULL_ROWS) and calls that ask
 // for the planes stay with them.

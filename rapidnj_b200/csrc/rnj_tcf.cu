@@ -35,9 +35,9 @@
 //
 // What bounds it.  Long alignments: the MMAs of a pair, 326 cycles per 256
 // columns with operands at rest, 343 with loads, 436 with the epilogue at work
-// (10,000 x 10,000 DNA call 1.007 -> 0.912 ms; the chip is at its 1,000 W limit
+// (10,000 x 10,000 DNA call 1.023 -> 0.930 ms; the chip is at its 1,000 W limit
 // there, 1.76 GHz).  Short ones: the epilogue, 69 warp instructions per 32 K2P
-// pairs (168 before: 50,000 x 1,000 call 7.55 -> 5.28 ms) at 0.46 issues a cycle
+// pairs (168 before: 50,000 x 1,000 call 7.55 -> 5.43 ms) at 0.46 issues a cycle
 // with four warps a scheduler, no pipe above a quarter of its rate; of what it
 // does, the stores cost 15 %, the table reads 9 %, each double operation about
 // 1.7 %.  Few tiles: set-up and one tile's latency (kSlices, tc_fused_kernel).
